@@ -620,7 +620,7 @@ int32_t gllmk_dequantize_i32_f32(gllmk_ctx ctx, const int32_t *c_dev, float *out
     if (m < 0 || n < 0) return fail(c, GLLMK_STATUS_INVALID_ARG, "dequantize: negative shape");
     if (activation < 0 || activation > 4) return fail(c, GLLMK_STATUS_UNSUPPORTED, "dequantize: activation %d", activation);
     DeviceGuard g(c->device);
-    return dequant_i32_launch(c, c_dev, out_dev, m, n, n, n, scale_a, scale_b, bias_dev, activation, static_cast<cudaStream_t>(stream));
+    return dequant_i32_launch(c, c_dev, out_dev, m, n, scale_a, scale_b, bias_dev, activation, static_cast<cudaStream_t>(stream));
 }
 
 int32_t gllmk_quantize_act_int8(gllmk_ctx ctx, const float *x_dev, int64_t rows, int64_t k, int64_t ldx, void *q_dev, int64_t ldq,
@@ -643,21 +643,7 @@ int32_t gllmk_w8a8_linear_f32(gllmk_ctx ctx, gllmk_weight wh, const float *x_dev
     if (activation < 0 || activation > 4) return fail(c, GLLMK_STATUS_UNSUPPORTED, "w8a8_linear: activation %d", activation);
     if (w->device != c->device) return fail(c, GLLMK_STATUS_INVALID_ARG, "weight lives on another device");
     DeviceGuard g(c->device);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // context scratch: [scale f32, amax u32 | pad to 256] [u8 activations m x k] [s32 products m x n]
-    const size_t ab = ((size_t)m * (size_t)w->k + 255) & ~(size_t)255, cb = (size_t)m * (size_t)w->n * sizeof(int32_t);
-    // (the context's device I/O buffer: the integer GEMM stages its tile images in the activation workspace itself)
-    int32_t rc = ensure_dev_io(c, 256 + ab + cb);
-    if (rc) return rc;
-    char *base = static_cast<char *>(c->dev_io);
-    float *scale = reinterpret_cast<float *>(base);
-    uint8_t *q = reinterpret_cast<uint8_t *>(base + 256);
-    int32_t *ci = reinterpret_cast<int32_t *>(base + 256 + ab);
-    rc = act_quant_i8_launch(c, x_dev, m, w->k, ldx, q, w->k, 128, scale, s);
-    if (!rc) rc = gemm_i8_launch(c, w, q, w->k, m, ci, w->n, s);
-    if (!rc) rc = dequant_i32_launch(c, ci, y_dev, m, w->n, w->n, ldy, 0.0f, scale_b, bias_dev, activation, s, scale,
-                                     static_cast<const int32_t *>(w->aux));
-    return rc;
+    return w8a8_linear_launch(c, w, x_dev, ldx, m, y_dev, ldy, scale_b, bias_dev, activation, static_cast<cudaStream_t>(stream));
 }
 
 int32_t gllmk_gemm_int8_host(gllmk_ctx ctx, const uint8_t *a, const int8_t *b_kn, int32_t *c_out, size_t m, size_t n, size_t k) {

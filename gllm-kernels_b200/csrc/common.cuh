@@ -184,9 +184,10 @@ int32_t gemv_fp4_launch(Ctx *c, const Weight *w, const float *x, int64_t xst, in
 // ---- gemm_i8.cu ----
 int32_t i8_weight_fill(Ctx *c, Weight *w, const int8_t *b_dev, int layout, cudaStream_t s);
 int32_t gemm_i8_launch(Ctx *c, const Weight *w, const uint8_t *a, int64_t lda, int m, int32_t *out, int64_t ldc, cudaStream_t s);
-int32_t dequant_i32_launch(Ctx *c, const int32_t *ci, float *out, int64_t m, int64_t n, int64_t ldc, int64_t ldo, float scale_a,
-                           float scale_b, const float *bias, int act, cudaStream_t s, const float *scale_a_dev = nullptr,
-                           const int32_t *colsum = nullptr);
+int32_t w8a8_linear_launch(Ctx *c, const Weight *w, const float *x, int64_t ldx, int m, float *y, int64_t ldy, float scale_b, const float *bias,
+                           int act, cudaStream_t s);
+int32_t dequant_i32_launch(Ctx *c, const int32_t *ci, float *out, int64_t m, int64_t n, float scale_a, float scale_b, const float *bias,
+                           int act, cudaStream_t s);
 // f32 activations -> per-tensor int8 (stored as q + offset); scale_dev: two words of device memory, [0] receives the scale
 int32_t act_quant_i8_launch(Ctx *c, const float *x, int64_t rows, int64_t k, int64_t ld, uint8_t *q, int64_t ldq, int offset,
                             float *scale_dev, cudaStream_t s);

@@ -12,6 +12,8 @@
 #include "common.cuh"
 #include "tc05.cuh"
 
+#include <type_traits>
+
 namespace gllmk {
 
 constexpr int I8_BM = 128, I8_BN = 256, I8_TILE = 16384;
@@ -34,11 +36,77 @@ struct I8Params {
     int row_tiles;
     int nks;            // k-steps of 128
     int m;
-    int32_t *c;         // [m, n] row-major, leading dimension ldc
+    void *c;            // [m, n] row-major, leading dimension ldc: s32 products, or (EPI) the finished f32 outputs
     int64_t ldc;
     int vec;
     int *status;
+    // EPI (a whole W8A8 linear layer): the epilogue of dequant_i32_kernel on the accumulator while it is in registers
+    const float *scale_a;   // device memory: written by the activation quantizer of the same stream
+    const int32_t *colsum;  // sum_k W[j, k]: the activations are stored as q + 128
+    const float *bias;      // nullptr: none
+    float scale_b;
+    int act;
 };
+
+// v / (1 + exp(-z)): SiLU with z = v; the tanh form of GELU, 0.5 v (1 + tanh(u)) = v / (1 + exp(-2u)), with z = 2u (and no
+// cancellation for negative u).  The quotient is Markstein's (q = v y, q += (v - q d) y, y an approximate 1 / d): no branch,
+// so the chains of a thread's 32 elements overlap; the compiler's IEEE division has one per element, and the fused
+// epilogue of gemm_i8_pair_kernel then took 134 us on W[11008, 4096] x 2048 (82 now; the product without it 72).
+__device__ __forceinline__ float sigmoid_times(float v, float z) {
+    const float d = 1.0f + expf(-z), y = __fdividef(1.0f, d), q = v * y;
+    return d < 1e37f ? fmaf(fmaf(-q, d, v), y, q) : q;  // exp overflows: y = 0, and the residual would be 0 * inf
+}
+// dequantize_i32_to_f32 (src/macros/matmul_x86_int8.rs:414-456, scalar tail semantics): (c as f32) * scale_a * scale_b
+// (+ bias[j]), then the activation of src/macros/gemm_epilogue.rs:131-152
+template <int ACT>
+__device__ __forceinline__ float i8_dequant(int32_t c, float scale_a, float scale_b, bool has_bias, float bias) {
+    float v = __fmul_rn(__fmul_rn((float)c, scale_a), scale_b);
+    if (has_bias) v = __fadd_rn(v, bias);
+    if (ACT == 1) v = v < 0.0f ? 0.0f : v;
+    else if (ACT == 2) v = sigmoid_times(v, v);
+    else if (ACT == 3) v = sigmoid_times(v, 2.0f * (0.7978845608f * (v + 0.044715f * v * v * v)));
+    return v;
+}
+// the activation as a compile-time constant (GELU and GEGLU share a formula)
+template <typename F>
+__device__ __forceinline__ void with_act(int act, F &&f) {
+    if (act == 0) f(std::integral_constant<int, 0>{});
+    else if (act == 1) f(std::integral_constant<int, 1>{});
+    else if (act == 2) f(std::integral_constant<int, 2>{});
+    else f(std::integral_constant<int, 3>{});
+}
+
+// One 32-row x 32-token block of accumulators (lane = weight row) made ready for the 32-bit store helper: the s32 bit
+// patterns as they are, or (EPI) the layer's f32 outputs.  In the linear layer the accumulator never goes to memory: as a
+// pass of its own over the s32 products this epilogue moved 8 bytes per output (W[11008, 4096] x 2048 tokens: 95 of 230 us).
+struct I8Lane {  // what a lane's weight row contributes (EPI)
+    float scale_a, bias;
+    int32_t off;  // 128 * colsum of the row: exact, the s32 range holds both terms for k < 66000
+};
+template <bool EPI>
+__device__ __forceinline__ I8Lane i8_lane(const I8Params &p, int64_t row) {
+    I8Lane l{0.0f, 0.0f, 0};
+    if constexpr (EPI) {
+        l.scale_a = *p.scale_a;
+        if (row < p.n) {
+            l.off = 128 * p.colsum[row];
+            if (p.bias) l.bias = p.bias[row];
+        }
+    }
+    return l;
+}
+template <bool EPI>
+__device__ __forceinline__ void i8_finish(const I8Params &p, const I8Lane &l, const uint32_t (&v)[32], float (&o)[32]) {
+    if constexpr (EPI) {
+        with_act(p.act, [&](auto act) {
+#pragma unroll
+            for (int j = 0; j < 32; j++) o[j] = i8_dequant<act.value>((int32_t)v[j] - l.off, l.scale_a, p.scale_b, p.bias != nullptr, l.bias);
+        });
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j++) o[j] = __uint_as_float(v[j]);
+    }
+}
 
 __device__ __forceinline__ void i8_bulk(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src),
@@ -70,6 +138,7 @@ __global__ void __launch_bounds__(256) repack_i8_kernel(const int8_t *__restrict
 // ---- u8 activations [m, k] (leading dimension lda, any alignment) -> tile images; grid (k-steps, token tiles of 128)
 __global__ void __launch_bounds__(256) stage_act_u8_kernel(const uint8_t *__restrict__ a, int64_t lda, int m, int64_t k,
                                                            uint8_t *__restrict__ xt) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const int ks = blockIdx.x, tile = blockIdx.y;
     uint8_t *dst = xt + ((size_t)tile * gridDim.x + ks) * I8_TILE;
 #pragma unroll
@@ -87,7 +156,7 @@ __global__ void __launch_bounds__(256) stage_act_u8_kernel(const uint8_t *__rest
 }
 
 // grid (groups of MT weight-row tiles, token tiles of 256); ntok = MMA N (multiple of 32, <= 256)
-template <int MT>
+template <int MT, bool EPI>
 __global__ void __launch_bounds__(I8_THREADS, 1) gemm_i8_kernel(const __grid_constant__ I8Params p, const int ntok) {
     constexpr int I8_STAGES = i8_stages<MT>(), I8_STAGE_BYTES = i8_stage_bytes<MT>();
     constexpr uint32_t TMEM_COLS = MT == 2 ? 512 : 256;
@@ -123,6 +192,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) gemm_i8_kernel(const __grid_con
         const int halves = (ntok + 127) / 128;
         const uint32_t bbytes = (uint32_t)ntok * 128u;
         const uint32_t hb[2] = {ntok > 128 ? (uint32_t)I8_TILE : bbytes, bbytes - (uint32_t)I8_TILE};
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the activation images are complete from here on
         for (int ks = 0; ks < p.nks; ks++) {
             const int s = ks % I8_STAGES;
             if (ks >= I8_STAGES && !tc::mbar_wait(empty + 8 * s, (uint32_t)((ks / I8_STAGES - 1) & 1), abort_flag)) {
@@ -173,18 +243,19 @@ __global__ void __launch_bounds__(I8_THREADS, 1) gemm_i8_kernel(const __grid_con
         }
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
+            asm volatile("griddepcontrol.wait;\n" ::: "memory");  // this thread reads the activation scale
             tc::fence_after_sync();
             // all MMAs have completed, so the stages are free: each warp stages its blocks in 4 KB of stage 0
             uint8_t *stage = smem_raw + (smem_s - tc::smem_u32(smem_raw)) + (warp - 2) * 4096;
             for (int i = 0; i < mt; i++) {
                 const int64_t row0 = (int64_t)(tile0 + i) * I8_BM;
+                const I8Lane l = i8_lane<EPI>(p, row0 + 32 * quad + lane);
                 for (int c = 32 * ((warp - 2) >> 2); c < ntok; c += 32 * (I8_EPI_WARPS / 4)) {
                     uint32_t v[32];
                     tc::tmem_ld32(tmem + ((uint32_t)(32 * quad) << 16) + 256u * (uint32_t)i + (uint32_t)c, v);
                     tc::tmem_ld_wait();
-                    float o[32];  // the s32 bit patterns travel through the 32-bit store helper unchanged
-#pragma unroll
-                    for (int j = 0; j < 32; j++) o[j] = __uint_as_float(v[j]);
+                    float o[32];
+                    i8_finish<EPI>(p, l, v, o);
                     tc::store_block_32x32<false>(p.c, p.ldc, row0 + 32 * quad, tok0 + c, p.n, p.m, o, stage, lane, p.vec);
                 }
             }
@@ -210,6 +281,7 @@ constexpr int I8P_STAGES = 6, I8P_STAGE_BYTES = 2 * I8_TILE, I8P_EPI_WARPS = 8;
 constexpr int I8P_THREADS = 64 + 32 * I8P_EPI_WARPS;
 constexpr size_t I8P_SMEM = (size_t)I8P_STAGES * I8P_STAGE_BYTES + (size_t)I8P_EPI_WARPS * 4096 + 1024;
 
+template <bool EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(I8P_THREADS, 1)
 gemm_i8_pair_kernel(const __grid_constant__ I8Params p, const int tok_tiles, const int x_tiles) {
     extern __shared__ uint8_t smem_raw[];
@@ -250,6 +322,7 @@ gemm_i8_pair_kernel(const __grid_constant__ I8Params p, const int tok_tiles, con
     if (warp == 0 && lane == 0) {
         // ---------------- copies: own weight rows, own half of the activation tile ----------------
         uint32_t g = 0;
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the activation images are complete from here on
         for (int t = pair; t < ntiles && !*abort_flag; t += npairs) {
             const int rp = t / tok_tiles, tt = t % tok_tiles;
             const int my_row_tile = 2 * rp + (int)rank, my_x_tile = 2 * tt + (int)rank;
@@ -332,6 +405,7 @@ gemm_i8_pair_kernel(const __grid_constant__ I8Params p, const int tok_tiles, con
         uint8_t *stage = smem_raw + (smem_s - tc::smem_u32(smem_raw)) + (size_t)I8P_STAGES * I8P_STAGE_BYTES + (size_t)(warp - 2) * 4096;
         const uint32_t accum_empty_leader = tc::map_to_cta(accum_empty, 0);
         uint32_t it = 0;
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");  // this thread reads the activation scale
         for (int t = pair; t < ntiles; t += npairs, it++) {
             const uint32_t acc = it & 1u;
             bool ok = !abort_s && tc::mbar_wait_cluster(accum_full + 8 * acc, (it >> 1) & 1u, abort_flag);
@@ -345,15 +419,15 @@ gemm_i8_pair_kernel(const __grid_constant__ I8Params p, const int tok_tiles, con
             const int rp = t / tok_tiles, tt = t % tok_tiles;
             const int64_t row0 = (int64_t)(2 * rp + (int)rank) * I8_BM + 32 * quad, tok0 = (int64_t)tt * I8_BN + 128 * half;
             const uint32_t tbase = tmem + ((uint32_t)(32 * quad) << 16) + 256u * acc + (uint32_t)(128 * half);
+            const I8Lane l = i8_lane<EPI>(p, row0 + lane);
 #pragma unroll 1
             for (int c = 0; c < 128; c += 32) {
                 uint32_t v[32];
                 tc::tmem_ld32(tbase + (uint32_t)c, v);
                 tc::tmem_ld_wait();
                 if (row0 < p.n && tok0 + c < p.m) {
-                    float o[32];  // the s32 bit patterns travel through the 32-bit store helper unchanged
-#pragma unroll
-                    for (int j = 0; j < 32; j++) o[j] = __uint_as_float(v[j]);
+                    float o[32];
+                    i8_finish<EPI>(p, l, v, o);
                     tc::store_block_32x32<false>(p.c, p.ldc, row0, tok0 + c, p.n, p.m, o, stage, lane, p.vec);
                 }
             }
@@ -371,30 +445,13 @@ gemm_i8_pair_kernel(const __grid_constant__ I8Params p, const int tok_tiles, con
     if (warp == 1) tc::tmem_dealloc_pair(tmem, 512);
 }
 
-// dequantize_i32_to_f32 (src/macros/matmul_x86_int8.rs:414-456, scalar tail semantics): (c as f32) * scale_a * scale_b
-// (+ bias[j]), then the activation of src/macros/gemm_epilogue.rs:131-152
-// scale_a_dev != nullptr: the activation scale is read from device memory (written by the activation quantizer of the
-// same stream).  colsum != nullptr: the activations were stored as q + 128 (unsigned), so 128 * sum_k B[k, j] is
-// taken off the integer result first — exact, the s32 range holds both terms for k < 66000.
-__global__ void __launch_bounds__(256) dequant_i32_kernel(const int32_t *__restrict__ c, float *__restrict__ out, int64_t n, int64_t ldc,
-                                                          int64_t ldo, float scale_a, float scale_b, const float *__restrict__ bias,
-                                                          int act, size_t total, const float *__restrict__ scale_a_dev,
-                                                          const int32_t *__restrict__ colsum) {
+// the epilogue as a pass of its own (gllmk_dequantize_i32_f32)
+__global__ void __launch_bounds__(256) dequant_i32_kernel(const int32_t *__restrict__ c, float *__restrict__ out, int64_t n, float scale_a,
+                                                          float scale_b, const float *__restrict__ bias, int act, size_t total) {
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
-    const int64_t i = (int64_t)(idx / (size_t)n), j = (int64_t)(idx % (size_t)n);
-    if (scale_a_dev) scale_a = *scale_a_dev;
-    int32_t ci = c[i * ldc + j];
-    if (colsum) ci -= 128 * colsum[j];
-    float v = __fmul_rn(__fmul_rn((float)ci, scale_a), scale_b);
-    if (bias) v = __fadd_rn(v, bias[j]);
-    if (act == 1) v = v < 0.0f ? 0.0f : v;
-    else if (act == 2) v = v / (1.0f + expf(-v));
-    else if (act == 3 || act == 4) {
-        const float inner = 0.7978845608f * (v + 0.044715f * v * v * v);
-        v = 0.5f * v * (1.0f + tanhf(inner));
-    }
-    out[i * ldo + j] = v;
+    const float b = bias ? bias[idx % (size_t)n] : 0.0f;
+    with_act(act, [&](auto a) { out[idx] = i8_dequant<a.value>(c[idx], scale_a, scale_b, bias != nullptr, b); });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -423,76 +480,207 @@ int32_t i8_weight_fill(Ctx *c, Weight *w, const int8_t *b_dev, int layout, cudaS
 
 // quantize_from_fp32 / QuantFormat::Int8PerTensor (src/compiler/quant_convert.rs:17-20,165-177): scale = max|x| / 127,
 // q = (x / scale).round().clamp(-128, 127) as i8 (round half away from zero; NaN, i.e. 0 / 0 for an all-zero tensor, -> 0).
-__global__ void __launch_bounds__(256) act_amax_kernel(const float *__restrict__ x, int64_t rows, int64_t k, int64_t ld, uint32_t *amax_bits) {
+//
+// Two passes, both bound by reading x (the second finds it in L2 up to ~100 MB): block maxima, then every block of the
+// second pass reduces the (at most AQ_PARTS) block maxima itself, under its own loads of x, so there is no atomic, no
+// cleared word and no launch in between.  x [2048, 4096] from a cold cache: 8 + 16 us (4-byte loads, an atomic maximum and a
+// byte image that a third pass turned into tile images: 24 + 41 + 9 us).
+constexpr int AQ_PARTS = 592;      // blocks of the first pass: four per SM
+constexpr int AQ_SCALE_OFF = 72;   // words of the context's small device scratch (behind its status word): scale, maximum
+constexpr int AQ_PART_OFF = 128;   // and the block maxima
+constexpr int AQ_ROWS = 8;         // rows (16-byte loads in flight) per thread of the second pass
+constexpr int AQ_SEG = 4096;       // elements a block takes at a time: four 16-byte loads per thread in flight
+
+__device__ __forceinline__ float max_abs4(float a, float4 v) {
+    // f32::max semantics: a NaN operand is ignored
+    return fmaxf(fmaxf(a, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+}
+__global__ void __launch_bounds__(256) act_amax_kernel(const float *__restrict__ x, int64_t rows, int64_t k, int64_t ld, int vec,
+                                                       float *__restrict__ partial) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    __shared__ float red[8];
+    const int64_t segs = (k + AQ_SEG - 1) / AQ_SEG, units = rows * segs;
     float a = 0.0f;
-    const int64_t total = rows * k;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const float v = fabsf(x[(i / k) * ld + i % k]);
-        if (v > a) a = v;  // f32::max semantics: a NaN operand is ignored
+    for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
+        const int64_t r = u / segs, c0 = (u - r * segs) * AQ_SEG;
+        const float *src = x + r * ld + c0;
+        const int n = (int)(k - c0 < AQ_SEG ? k - c0 : AQ_SEG);
+        if (vec) {
+            float4 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int c = 4 * ((int)threadIdx.x + 256 * i);
+                v[i] = c < n ? __ldg(reinterpret_cast<const float4 *>(src + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) a = max_abs4(a, v[i]);
+        } else {
+#pragma unroll 8
+            for (int c = threadIdx.x; c < n; c += 256) a = fmaxf(a, fabsf(src[c]));
+        }
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(amax_bits, __float_as_uint(a));  // non-negative floats order like their bits
-}
-__global__ void __launch_bounds__(256) act_quant_i8_kernel(const float *__restrict__ x, int64_t rows, int64_t k, int64_t ld, uint8_t *__restrict__ q,
-                                                           int64_t ldq, int offset, const uint32_t *amax_bits, float *scale_out) {
-    const float scale = __fdiv_rn(__uint_as_float(*amax_bits), 127.0f);
-    const int64_t total = rows * k;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / k, cidx = i % k;
-        float v = roundf(__fdiv_rn(x[r * ld + cidx], scale));
-        if (v != v) v = 0.0f;
-        v = fminf(fmaxf(v, -128.0f), 127.0f);
-        q[r * ldq + cidx] = (uint8_t)((int)v + offset);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 1; i < 8; i++) a = fmaxf(a, red[i]);
+        partial[blockIdx.x] = a;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
 }
 
-int32_t act_quant_i8_launch(Ctx *c, const float *x, int64_t rows, int64_t k, int64_t ld, uint8_t *q, int64_t ldq, int offset,
-                            float *scale_dev, cudaStream_t s) {
-    // the running maximum lives next to the caller's scale word: [scale f32][amax bits u32]
-    uint32_t *amax = reinterpret_cast<uint32_t *>(scale_dev) + 1;
-    GK_CUDA(c, cudaMemsetAsync(amax, 0, sizeof(uint32_t), s));
-    const int64_t total = rows * k;
-    const unsigned grid = (unsigned)((total + 1023) / 1024 > 1184 ? 1184 : (total + 1023) / 1024);
-    act_amax_kernel<<<grid, 256, 0, s>>>(x, rows, k, ld, amax);
-    act_quant_i8_kernel<<<grid, 256, 0, s>>>(x, rows, k, ld, q, ldq, offset, amax, scale_dev);
+// IMG: the quantized activations (as q + 128) go straight into the tile images the integer GEMM copies (128 tokens x 128 k,
+// swizzled); otherwise to q [rows, ldq].  A warp takes 128 k of a row (16 bytes in, 4 bytes out per lane: whole lines both
+// ways, an image row is one 128-byte line), a thread AQ_ROWS rows, all loaded first.  grid (k / 128, rows / (8 AQ_ROWS)).  Tokens past the last one are
+// not written: what an image holds there only reaches accumulator columns that are never stored.
+template <bool IMG>
+__global__ void __launch_bounds__(256) act_quant_i8_kernel(const float *__restrict__ x, int64_t rows, int64_t k, int64_t ld, int vec,
+                                                           uint8_t *__restrict__ q, int64_t ldq, int qvec, int offset,
+                                                           const float *__restrict__ partial, int nparts, float *scale_out) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    __shared__ float red[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t k0 = (int64_t)blockIdx.x * 128 + 4 * lane;
+    float4 v[AQ_ROWS];
+#pragma unroll
+    for (int i = 0; i < AQ_ROWS; i++) {
+        const int64_t r = (int64_t)blockIdx.y * (8 * AQ_ROWS) + 8 * i + warp;
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < rows) {
+            const float *src = x + r * ld + k0;
+            if (vec && k0 < k) v[i] = __ldg(reinterpret_cast<const float4 *>(src));
+            else if (!vec) {
+                if (k0 < k) v[i].x = src[0];
+                if (k0 + 1 < k) v[i].y = src[1];
+                if (k0 + 2 < k) v[i].z = src[2];
+                if (k0 + 3 < k) v[i].w = src[3];
+            }
+        }
+    }
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the block maxima are complete from here on
+    float a = 0.0f;
+    for (int i = threadIdx.x; i < nparts; i += 256) a = fmaxf(a, __ldcg(partial + i));
+#pragma unroll
+    for (int o = 16; o; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
+    if (lane == 0) red[warp] = a;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; i++) a = fmaxf(a, red[i]);
+    const float scale = __fdiv_rn(a, 127.0f);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+        scale_out[0] = scale;
+        scale_out[1] = a;
+    }
+    // f / scale, correctly rounded: one reciprocal for all elements and two of Markstein's corrections (the first makes the
+    // quotient faithful, the second exact); scales so small or large that a step could leave the normal range divide
+    const bool fast = scale > 1e-30f && scale < 1e30f;
+    const float y = fast ? __frcp_rn(scale) : 0.0f;
+    const auto quant = [&](float f) -> uint32_t {
+        if (fast) {
+            float d = f * y;
+            d = fmaf(fmaf(-d, scale, f), y, d);
+            f = fmaf(fmaf(-d, scale, f), y, d);
+        } else {
+            f = __fdiv_rn(f, scale);
+        }
+        f = roundf(f);
+        if (f != f) f = 0.0f;
+        f = fminf(fmaxf(f, -128.0f), 127.0f);
+        return (uint32_t)((int)f + offset) & 0xFFu;
+    };
+#pragma unroll
+    for (int i = 0; i < AQ_ROWS; i++) {
+        const int64_t r = (int64_t)blockIdx.y * (8 * AQ_ROWS) + 8 * i + warp;
+        if (r >= rows) continue;
+        const uint32_t w = quant(v[i].x) | (quant(v[i].y) << 8) | (quant(v[i].z) << 16) | (quant(v[i].w) << 24);
+        if (IMG) {
+            uint8_t *dst = q + ((size_t)(r >> 7) * gridDim.x + blockIdx.x) * I8_TILE;
+            *reinterpret_cast<uint32_t *>(dst + tc::sw128_offset((int)(r & 127), lane >> 2) + 4 * (lane & 3)) = w;
+        } else if (qvec && k0 + 3 < k) {
+            *reinterpret_cast<uint32_t *>(q + r * ldq + k0) = w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (k0 + j < k) q[r * ldq + k0 + j] = (uint8_t)(w >> (8 * j));
+        }
+    }
+}
+
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_after(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+    // programmatic launch: starts as soon as every block of the kernel in front has issued griddepcontrol.launch_dependents
+    // (and orders its own reads after it with griddepcontrol.wait)
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
+// img: q is the tile images of the integer GEMM (ldq unused), otherwise [rows, ldq] bytes
+static int32_t act_quant(Ctx *c, const float *x, int64_t rows, int64_t k, int64_t ld, uint8_t *q, int64_t ldq, int offset, bool img,
+                         float *scale_dev, cudaStream_t s) {
+    float *partial = reinterpret_cast<float *>(c->status_dev) + AQ_PART_OFF;
+    const int vec = (((uintptr_t)x & 15) == 0 && ld % 4 == 0 && k % 4 == 0) ? 1 : 0;
+    const int qvec = (((uintptr_t)q & 3) == 0 && ldq % 4 == 0) ? 1 : 0;
+    // contiguous rows are one long row to the maximum
+    const int64_t ar = ld == k ? 1 : rows, ak = ld == k ? rows * k : k;
+    const int64_t units = ar * ((ak + AQ_SEG - 1) / AQ_SEG);
+    const int parts = (int)(units < AQ_PARTS ? units : AQ_PARTS);
+    act_amax_kernel<<<(unsigned)parts, 256, 0, s>>>(x, ar, ak, ld, vec, partial);
     GK_CUDA(c, cudaGetLastError());
+    // row groups beyond the grid's y limit: launches of their own (each writes the same scale)
+    const int64_t step = (int64_t)65534 * 8 * AQ_ROWS;  // a multiple of the 128 rows of an image
+    for (int64_t r0 = 0; r0 < rows; r0 += step) {
+        const int64_t nr = rows - r0 < step ? rows - r0 : step;
+        const dim3 grid((unsigned)((k + 127) / 128), (unsigned)((nr + 8 * AQ_ROWS - 1) / (8 * AQ_ROWS)));
+        uint8_t *dst = img ? q + (size_t)(r0 >> 7) * ((size_t)(k + 127) / 128) * I8_TILE : q + r0 * ldq;
+        GK_CUDA(c, img ? launch_after(act_quant_i8_kernel<true>, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, partial, parts, scale_dev)
+                       : launch_after(act_quant_i8_kernel<false>, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, partial, parts, scale_dev));
+    }
     return GLLMK_STATUS_OK;
 }
+int32_t act_quant_i8_launch(Ctx *c, const float *x, int64_t rows, int64_t k, int64_t ld, uint8_t *q, int64_t ldq, int offset,
+                            float *scale_dev, cudaStream_t s) {
+    return act_quant(c, x, rows, k, ld, q, ldq, offset, false, scale_dev, s);
+}
 
-template <int MT>
+template <int MT, bool EPI>
 static int32_t i8_launch_mt(Ctx *c, const I8Params &p, dim3 grid, int ntok, cudaStream_t s) {
     static bool attr_set[64] = {};  // function attributes are per device
     const int dev_slot = c->device & 63;
     if (!attr_set[dev_slot]) {
-        GK_CUDA(c, cudaFuncSetAttribute(gemm_i8_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)i8_smem<MT>()));
+        GK_CUDA(c, cudaFuncSetAttribute(gemm_i8_kernel<MT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)i8_smem<MT>()));
         attr_set[dev_slot] = true;
     }
-    gemm_i8_kernel<MT><<<grid, I8_THREADS, i8_smem<MT>(), s>>>(p, ntok);
-    GK_CUDA(c, cudaGetLastError());
+    GK_CUDA(c, launch_after(gemm_i8_kernel<MT, EPI>, grid, I8_THREADS, i8_smem<MT>(), s, p, ntok));
     return GLLMK_STATUS_OK;
 }
 
-int32_t gemm_i8_launch(Ctx *c, const Weight *w, const uint8_t *a, int64_t lda, int m, int32_t *out, int64_t ldc, cudaStream_t s) {
+// Activation images a launch over m tokens reads: 128 tokens each, pairs of them when the token tile is 256 wide
+static int i8_act_tiles(int m) { return m > 128 ? 2 * ((m + I8_BN - 1) / I8_BN) : 1; }
+
+// The product from the activation images in the context's scratch (written by the kernel just launched on `s`); p holds the
+// output and, with EPI, the epilogue's operands.
+template <bool EPI>
+static int32_t i8_product(Ctx *c, const Weight *w, I8Params p, int m, cudaStream_t s) {
     const int ntok = m > 128 ? I8_BN : (m + 31) / 32 * 32;
     const int mtiles = (m + I8_BN - 1) / I8_BN;
-    const int atiles = ntok > 128 ? 2 * mtiles : 1;
-    I8Params p{};
     p.w = static_cast<const uint8_t *>(w->qs);
+    p.xt = static_cast<const uint8_t *>(c->act);
     p.n = w->n;
     p.row_tiles = (int)(w->n_pad / I8_BM);
     p.nks = (int)(w->k_pad / 128);
     p.m = m;
-    p.c = out;
-    p.ldc = ldc;
-    p.vec = (((uintptr_t)out & 15) == 0 && (ldc * 4) % 16 == 0) ? 1 : 0;
+    p.vec = (((uintptr_t)p.c & 15) == 0 && (p.ldc * 4) % 16 == 0) ? 1 : 0;
     p.status = c->status_dev;
-    int32_t rc = ensure_act(c, (size_t)atiles * p.nks * I8_TILE);
-    if (rc) return rc;
-    p.xt = static_cast<const uint8_t *>(c->act);
-    stage_act_u8_kernel<<<dim3((unsigned)p.nks, (unsigned)atiles), 256, 0, s>>>(a, lda, m, w->k, static_cast<uint8_t *>(c->act));
-    GK_CUDA(c, cudaGetLastError());
     // estimated times in k-steps of a 128 x 256 tile (waves x (k-steps per CTA x relative step cost + a fixed prologue /
     // epilogue worth ~8 steps)): one row tile per CTA, two row tiles per CTA (a third fewer bytes per MAC), CTA pairs
     // (half the bytes per MAC of one tile per CTA; measured 0.82 of the two-tile form on W[11008, 4096] x 2048, 1.06 x 512)
@@ -502,7 +690,7 @@ int32_t gemm_i8_launch(Ctx *c, const Weight *w, const uint8_t *a, int64_t lda, i
     const int half_sms = c->sm_count / 2 > 0 ? c->sm_count / 2 : 1;
     const double tp = (double)((mtiles * pairs + half_sms - 1) / half_sms) * (p.nks * 0.6 + 8.0);
     if (m > 128 && (c->gemm_i8_pair == 2 || (c->gemm_i8_pair == 1 && tp < 0.9 * (t1 < t2 ? t1 : t2)))) {
-        const void *fn = (const void *)gemm_i8_pair_kernel;
+        const void *fn = (const void *)gemm_i8_pair_kernel<EPI>;
         static int pairs_resident[64] = {};  // per device: CTA pairs resident at once (0 = not yet asked)
         const int dev_slot = c->device & 63;
         if (!pairs_resident[dev_slot]) {
@@ -525,22 +713,52 @@ int32_t gemm_i8_launch(Ctx *c, const Weight *w, const uint8_t *a, int64_t lda, i
             }
             pairs_resident[dev_slot] = nclusters < c->sm_count / 2 ? nclusters : c->sm_count / 2;
         }
-        const int ntiles = ((p.row_tiles + 1) / 2) * mtiles;
+        const int ntiles = pairs * mtiles;
         const int npairs = ntiles < pairs_resident[dev_slot] ? ntiles : pairs_resident[dev_slot];
-        gemm_i8_pair_kernel<<<dim3(2u * (unsigned)npairs), I8P_THREADS, I8P_SMEM, s>>>(p, mtiles, atiles);
-        GK_CUDA(c, cudaGetLastError());
+        GK_CUDA(c, launch_after(gemm_i8_pair_kernel<EPI>, dim3(2u * (unsigned)npairs), I8P_THREADS, I8P_SMEM, s, p, mtiles, i8_act_tiles(m)));
         return GLLMK_STATUS_OK;
     }
-    if (ntok > 128 && t2 < t1) return i8_launch_mt<2>(c, p, dim3((unsigned)pairs, (unsigned)mtiles), ntok, s);
-    return i8_launch_mt<1>(c, p, dim3((unsigned)p.row_tiles, (unsigned)mtiles), ntok, s);
+    if (ntok > 128 && t2 < t1) return i8_launch_mt<2, EPI>(c, p, dim3((unsigned)pairs, (unsigned)mtiles), ntok, s);
+    return i8_launch_mt<1, EPI>(c, p, dim3((unsigned)p.row_tiles, (unsigned)mtiles), ntok, s);
 }
 
-int32_t dequant_i32_launch(Ctx *c, const int32_t *ci, float *out, int64_t m, int64_t n, int64_t ldc, int64_t ldo, float scale_a,
-                           float scale_b, const float *bias, int act, cudaStream_t s, const float *scale_a_dev, const int32_t *colsum) {
+int32_t gemm_i8_launch(Ctx *c, const Weight *w, const uint8_t *a, int64_t lda, int m, int32_t *out, int64_t ldc, cudaStream_t s) {
+    const int nks = (int)(w->k_pad / 128), atiles = i8_act_tiles(m);
+    int32_t rc = ensure_act(c, (size_t)atiles * nks * I8_TILE);
+    if (rc) return rc;
+    stage_act_u8_kernel<<<dim3((unsigned)nks, (unsigned)atiles), 256, 0, s>>>(a, lda, m, w->k, static_cast<uint8_t *>(c->act));
+    GK_CUDA(c, cudaGetLastError());
+    I8Params p{};
+    p.c = out;
+    p.ldc = ldc;
+    return i8_product<false>(c, w, p, m, s);
+}
+
+// A whole linear layer: per-tensor quantization of x into the GEMM's tile images, the product, the f32 epilogue on the
+// accumulator.  Three launches, x read twice, y written once.
+int32_t w8a8_linear_launch(Ctx *c, const Weight *w, const float *x, int64_t ldx, int m, float *y, int64_t ldy, float scale_b, const float *bias,
+                           int act, cudaStream_t s) {
+    int32_t rc = ensure_act(c, (size_t)i8_act_tiles(m) * (size_t)(w->k_pad / 128) * I8_TILE);
+    if (rc) return rc;
+    float *scale = reinterpret_cast<float *>(c->status_dev) + AQ_SCALE_OFF;
+    rc = act_quant(c, x, m, w->k, ldx, static_cast<uint8_t *>(c->act), 0, 128, true, scale, s);
+    if (rc) return rc;
+    I8Params p{};
+    p.c = y;
+    p.ldc = ldy;
+    p.scale_a = scale;
+    p.colsum = static_cast<const int32_t *>(w->aux);
+    p.bias = bias;
+    p.scale_b = scale_b;
+    p.act = act;
+    return i8_product<true>(c, w, p, m, s);
+}
+
+int32_t dequant_i32_launch(Ctx *c, const int32_t *ci, float *out, int64_t m, int64_t n, float scale_a, float scale_b, const float *bias,
+                           int act, cudaStream_t s) {
     const size_t total = (size_t)m * (size_t)n;
     if (total == 0) return GLLMK_STATUS_OK;
-    dequant_i32_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(ci, out, n, ldc, ldo, scale_a, scale_b, bias, act, total, scale_a_dev,
-                                                                      colsum);
+    dequant_i32_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(ci, out, n, scale_a, scale_b, bias, act, total);
     GK_CUDA(c, cudaGetLastError());
     return GLLMK_STATUS_OK;
 }

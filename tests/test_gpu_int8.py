@@ -192,3 +192,38 @@ def test_w8a8_linear_against_the_reference_pipeline(gk, K, oracle, m, n, k, act)
     else:
         assert np.allclose(y, ref, rtol=2e-6, atol=1e-7)
     w.free()
+
+
+@pytest.mark.parametrize("m,n,k,act,pair,mag", [(31, 129, 127, 0, 1, 1.0), (33, 260, 4098, 2, 1, 1.0), (129, 128, 132, 1, 2, 1.0), (257, 300, 640, 3, 2, 1.0),
+                                                (513, 513, 384, 0, 2, 1.0), (65, 64, 256, 0, 1, 1e-33), (128, 140, 260, 4, 0, 1e31)])
+def test_w8a8_linear_fused_epilogue_edges(gk, K, oracle, m, n, k, act, pair, mag):
+    """The linear layer quantizes straight into the GEMM's tile images and finishes on the accumulator: token and row counts
+    around the tiles of every kernel form, k that is no multiple of the 16-byte loads, a strided x, scales outside the range of
+    the reciprocal path.  Without an activation function bit-exact; SiLU / GELU: expf is within 2 ulp and its argument's
+    rounding is amplified by |v| < 90 (2 * 90 * 2^-24 = 1.1e-5 relative at most, where the output has all but vanished)."""
+    import torch
+    rng = np.random.default_rng(m + n + k)
+    x = (rng.standard_normal((m, k)) * 2.0 * mag).astype(np.float32)
+    b = rng.integers(-128, 128, size=(k, n), dtype=np.int8)
+    bias = rng.standard_normal(n).astype(np.float32)
+    scale_b = np.float32(0.013 / (mag * 100 * np.sqrt(k)))
+    wide = torch.zeros((m, k + 4), device="cuda")
+    wide[:, :k] = torch.from_numpy(x).cuda()
+    w = K.upload_int8(b, layout_kn=True)
+    q, s = oracle.quantize_int8_per_tensor(x)
+    c = (q.astype(np.int64) @ b.astype(np.int64)).astype(np.float32)
+    v = (c * np.float32(s)) * scale_b + bias
+    K.set("gemm_i8_pair", pair)
+    try:
+        y = K.w8a8_linear(w, wide[:, :k], float(scale_b), bias=torch.from_numpy(bias).cuda(), activation=act).cpu().numpy()
+        assert K.status() == 0
+    finally:
+        K.set("gemm_i8_pair", 1)
+    if act == 0:
+        assert np.array_equal(y.view(np.uint32), v.view(np.uint32))
+    else:
+        v64 = v.astype(np.float64)
+        z = v64 if act == 2 else 2 * 0.7978845608 * (v64 + 0.044715 * v64 ** 3)
+        ref = np.maximum(v64, 0) if act == 1 else v64 / (1 + np.exp(-z))
+        assert np.allclose(y, ref, rtol=1.1e-5, atol=1e-7)
+    w.free()
