@@ -2,6 +2,7 @@
 // here, before any launch; nothing below throws.
 #include <cuda_bf16.h>
 
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -53,14 +54,108 @@ int32_t ensure_cnt(Ctx *c, size_t bytes) {
     return GLLMK_STATUS_OK;
 }
 int32_t ensure_pin(Ctx *c, size_t bytes) { return grow(c, &c->pin, &c->pin_bytes, bytes, true); }
+int32_t ensure_host_word(Ctx *c) {
+    if (!c->host_word) GK_CUDA(c, cudaMallocHost(&c->host_word, 64));
+    if (!c->host_word_ready) GK_CUDA(c, cudaEventCreateWithFlags(&c->host_word_ready, cudaEventDisableTiming));
+    return GLLMK_STATUS_OK;
+}
 int32_t ensure_dev_io(Ctx *c, size_t bytes) { return grow(c, &c->dev_io, &c->dev_io_bytes, bytes, false); }
+
+// ---- device memory of weights ----
+// cudaMalloc and cudaFree each cost tens to hundreds of microseconds and cudaFree waits for the device, which is nothing for a
+// model's weights but most of the time of a call whose activations are quantized and uploaded like a weight
+// (gllmk_gemm_fp4: W[14336, 4096] x 2048 tokens 850 - 1360 us, 600 of them here).  Freed buffers of up to 64 MB therefore stay
+// with the library, at most 128 MB per device, until the last context of the device is freed or an allocation fails.  A buffer
+// that is taken again may still be read by kernels its last owner launched, on any stream: the taker waits for the device once
+// (an upload from device memory has to anyway).
+constexpr size_t POOL_MAX_BLOCK = (size_t)64 << 20, POOL_MAX_BYTES = (size_t)128 << 20;
+struct WeightPool {
+    struct Block { void *p; size_t bytes; };
+    std::mutex mu;
+    std::vector<Block> blocks;  // oldest first
+    size_t held = 0;
+    int contexts = 0;
+};
+static WeightPool &pool_of(int device) {
+    static WeightPool *pools = new WeightPool[64];  // never destroyed: weights may be freed while the process ends
+    return pools[device & 63];
+}
+// sizes are rounded up to an eighth of a power of two, so that token counts that differ a little share buffers
+static size_t pool_size(size_t bytes) {
+    if (bytes > POOL_MAX_BLOCK) return bytes;
+    size_t step = 4096;
+    while (step * 8 < bytes) step *= 2;
+    return (bytes + step - 1) / step * step;
+}
+static void pool_trim(int device) {
+    WeightPool &p = pool_of(device);
+    std::lock_guard<std::mutex> l(p.mu);
+    for (const WeightPool::Block &b : p.blocks) cudaFree(b.p);
+    p.blocks.clear();
+    p.held = 0;
+}
+// A buffer of at least *bytes (set to its size).  *waited: the device has been waited for.
+static cudaError_t pool_take(int device, size_t *bytes, void **out, bool *waited) {
+    *bytes = pool_size(*bytes);
+    *out = nullptr;
+    WeightPool &p = pool_of(device);
+    {
+        std::lock_guard<std::mutex> l(p.mu);
+        for (size_t i = p.blocks.size(); i-- > 0;)
+            if (p.blocks[i].bytes == *bytes) {
+                *out = p.blocks[i].p;
+                p.blocks.erase(p.blocks.begin() + (ptrdiff_t)i);
+                p.held -= *bytes;
+                break;
+            }
+    }
+    if (*out) {
+        const cudaError_t e = cudaDeviceSynchronize();
+        if (e == cudaSuccess) *waited = true;
+        else cudaFree(*out), *out = nullptr;
+        return e;
+    }
+    cudaError_t e = cudaMalloc(out, *bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        pool_trim(device);
+        e = cudaMalloc(out, *bytes);
+    }
+    return e;
+}
+static void pool_put(int device, void *ptr, size_t bytes) {
+    if (!ptr) return;
+    WeightPool &p = pool_of(device);
+    std::lock_guard<std::mutex> l(p.mu);
+    if (bytes > POOL_MAX_BLOCK || p.contexts == 0) {
+        cudaFree(ptr);
+        return;
+    }
+    while (p.held + bytes > POOL_MAX_BYTES) {
+        cudaFree(p.blocks.front().p);
+        p.held -= p.blocks.front().bytes;
+        p.blocks.erase(p.blocks.begin());
+    }
+    p.blocks.push_back({ptr, bytes});
+    p.held += bytes;
+}
+
+// Device buffers of a weight whose plane sizes are set: one allocation, the auxiliary plane behind the main one.
+static int32_t weight_buffers(Ctx *c, Weight *w, bool *waited) {
+    const size_t aux_off = (w->qs_bytes + 255) & ~(size_t)255;
+    w->alloc_bytes = aux_off + w->aux_bytes;
+    const cudaError_t e = pool_take(c->device, &w->alloc_bytes, &w->qs, waited);
+    if (e != cudaSuccess) return cuda_fail(c, e, "cudaMalloc(weight)");
+    if (w->aux_bytes) w->aux = static_cast<char *>(w->qs) + aux_off;
+    return GLLMK_STATUS_OK;
+}
 
 // QuantType::block_size / block_bytes: read from the format descriptor table (quant_format.cuh)
 static int block_size_of(int qt, int mx) { return quant_format(qt, mx).block_size; }
 static int block_bytes_of(int qt, int mx) { return quant_format(qt, mx).block_bytes; }
 
 // Creates the handle and its device buffers for an n x k matrix of type qt (no data yet).
-static int32_t weight_alloc(Ctx *c, int32_t qt, int64_t n, int64_t k, int32_t mx_block, float global, Weight **out) {
+static int32_t weight_alloc(Ctx *c, int32_t qt, int64_t n, int64_t k, int32_t mx_block, float global, Weight **out, bool *waited) {
     if (qt != GLLMK_QUANT_Q4K && qt != GLLMK_QUANT_Q8_0 && qt != GLLMK_QUANT_MXFP4 && qt != GLLMK_QUANT_NVFP4 && !raw_format(qt))
         return fail(c, GLLMK_STATUS_UNSUPPORTED, "unknown quant type %d", qt);
     if (qt == GLLMK_QUANT_MXFP4 && mx_block != 32)
@@ -102,12 +197,10 @@ static int32_t weight_alloc(Ctx *c, int32_t qt, int64_t n, int64_t k, int32_t mx
         w->qs_bytes = (size_t)w->n_pad * (w->k_pad / 2);
         w->aux_bytes = (size_t)w->n_pad * (w->k_pad / (qt == GLLMK_QUANT_NVFP4 ? 16 : 32));
     }
-    cudaError_t e = cudaMalloc(&w->qs, w->qs_bytes);
-    if (e == cudaSuccess && w->aux_bytes) e = cudaMalloc(&w->aux, w->aux_bytes);
-    if (e != cudaSuccess) {
-        if (w->qs) cudaFree(w->qs);
+    const int32_t rc = weight_buffers(c, w, waited);
+    if (rc) {
         delete w;
-        return cuda_fail(c, e, "cudaMalloc(weight)");
+        return rc;
     }
     *out = w;
     return GLLMK_STATUS_OK;
@@ -116,13 +209,13 @@ static int32_t weight_alloc(Ctx *c, int32_t qt, int64_t n, int64_t k, int32_t mx
 static void weight_destroy(Weight *w) {
     if (!w) return;
     DeviceGuard g(w->device);
-    if (w->qs) cudaFree(w->qs);
-    if (w->aux) cudaFree(w->aux);
+    pool_put(w->device, w->qs, w->alloc_bytes);
     delete w;
 }
 
-// blocks/scales: host or device according to on_device.  Synchronous: returns once repacked.
-static int32_t weight_fill(Ctx *c, Weight *w, const void *blocks, const void *scales, bool on_device) {
+// blocks/scales: host or device according to on_device.  Synchronous: returns once repacked.  waited: the device has been
+// waited for since the call began.
+static int32_t weight_fill(Ctx *c, Weight *w, const void *blocks, const void *scales, bool on_device, bool waited) {
     const size_t raw = (w->qt == GLLMK_QUANT_MXFP4 && scales) ? (size_t)w->n * (w->k / 2) : (size_t)w->ref_bytes;
     const size_t sraw = (w->qt == GLLMK_QUANT_MXFP4 && scales) ? (size_t)w->n * (w->k / 32) : 0;
     const void *bdev = blocks, *sdev = scales;
@@ -140,7 +233,7 @@ static int32_t weight_fill(Ctx *c, Weight *w, const void *blocks, const void *sc
         if (((uintptr_t)blocks & 15) != 0) return fail(c, GLLMK_STATUS_INVALID_ARG, "device block pointer must be 16-byte aligned");
         // The caller's kernels that produce the blocks run on streams this library does not know: the repack (on the
         // context's own non-blocking stream) must not start before they have finished.  Load-time call: wait for the device.
-        GK_CUDA(c, cudaDeviceSynchronize());
+        if (!waited) GK_CUDA(c, cudaDeviceSynchronize());
     }
     int32_t rc = repack_upload(c, w, bdev, sdev, c->stream);
     cudaError_t e = cudaStreamSynchronize(c->stream);
@@ -220,6 +313,11 @@ int32_t gllmk_ctx_create(int32_t device, gllmk_ctx *out) {
         delete c;
         return GLLMK_STATUS_RUNTIME_ERROR;
     }
+    {
+        WeightPool &pool = pool_of(device);
+        std::lock_guard<std::mutex> l(pool.mu);
+        pool.contexts++;
+    }
     *out = c;
     return GLLMK_STATUS_OK;
 }
@@ -229,6 +327,13 @@ void gllmk_ctx_free(gllmk_ctx ctx) {
     Ctx *c = static_cast<Ctx *>(ctx);
     DeviceGuard g(c->device);
     cudaDeviceSynchronize();
+    bool last;
+    {
+        WeightPool &pool = pool_of(c->device);
+        std::lock_guard<std::mutex> l(pool.mu);
+        last = --pool.contexts == 0;
+    }
+    if (last) pool_trim(c->device);  // nobody is left to take the buffers again
     if (c->ws) cudaFree(c->ws);
     if (c->red) cudaFree(c->red);
     if (c->act) cudaFree(c->act);
@@ -236,6 +341,8 @@ void gllmk_ctx_free(gllmk_ctx ctx) {
     if (c->status_dev) cudaFree(c->status_dev);
     if (c->dev_io) cudaFree(c->dev_io);
     if (c->pin) cudaFreeHost(c->pin);
+    if (c->host_word) cudaFreeHost(c->host_word);
+    if (c->host_word_ready) cudaEventDestroy(c->host_word_ready);
     if (c->batch_exec) cudaGraphExecDestroy(c->batch_exec);
     for (cudaEvent_t e : c->events) cudaEventDestroy(e);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
@@ -308,9 +415,10 @@ int32_t gllmk_weight_upload(gllmk_ctx ctx, int32_t quant_type, int64_t n, int64_
         return fail(c, GLLMK_STATUS_INVALID_ARG, "scales must be NULL unless the type is MXFP4 (split form)");
     DeviceGuard g(c->device);
     Weight *w = nullptr;
-    int32_t rc = weight_alloc(c, quant_type, n, k, mx_block, global_scale, &w);
+    bool waited = false;
+    int32_t rc = weight_alloc(c, quant_type, n, k, mx_block, global_scale, &w, &waited);
     if (rc) return rc;
-    rc = weight_fill(c, w, blocks, scales, src_on_device != 0);
+    rc = weight_fill(c, w, blocks, scales, src_on_device != 0, waited);
     if (rc) { weight_destroy(w); return rc; }
     *out = w;
     return GLLMK_STATUS_OK;
@@ -555,15 +663,15 @@ static int32_t int8_weight_create(Ctx *c, int64_t n, int64_t k, const int8_t *b,
     w->ref_bytes = (uint64_t)n * (uint64_t)k;
     w->qs_bytes = (size_t)w->n_pad * (size_t)w->k_pad;
     w->aux_bytes = (size_t)n * sizeof(int32_t);  // column sums of B (zero-point correction of the f32 activation path)
-    cudaError_t e = cudaMalloc(&w->qs, w->qs_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&w->aux, w->aux_bytes);
-    if (e != cudaSuccess) {
-        if (w->qs) cudaFree(w->qs);
+    bool waited = false;
+    int32_t rc = weight_buffers(c, w, &waited);
+    if (rc) {
         delete w;
-        return cuda_fail(c, e, "cudaMalloc(int8 weight)");
+        return rc;
     }
     const int8_t *bdev = b;
     void *stage = nullptr;
+    cudaError_t e = cudaSuccess;
     if (!on_device) {
         e = cudaMalloc(&stage, (size_t)n * (size_t)k);
         if (e == cudaSuccess) e = cudaMemcpyAsync(stage, b, (size_t)n * (size_t)k, cudaMemcpyHostToDevice, c->stream);
@@ -573,10 +681,10 @@ static int32_t int8_weight_create(Ctx *c, int64_t n, int64_t k, const int8_t *b,
             return cuda_fail(c, e, "upload(int8 weight)");
         }
         bdev = static_cast<const int8_t *>(stage);
-    } else {
+    } else if (!waited) {
         (void)cudaDeviceSynchronize();  // the kernels that produced b ran on the caller's streams (see weight_fill)
     }
-    int32_t rc = i8_weight_fill(c, w, bdev, layout, c->stream);
+    rc = i8_weight_fill(c, w, bdev, layout, c->stream);
     e = cudaStreamSynchronize(c->stream);
     if (stage) cudaFree(stage);
     if (!rc && e != cudaSuccess) rc = cuda_fail(c, e, "repack(int8 weight)");
@@ -966,9 +1074,10 @@ static int32_t family_matmul(gllmk_ctx ctx, const uint8_t *wb, const float *inpu
     if (n > 0x7fffffffu) return fail(c, GLLMK_STATUS_INVALID_ARG, "n too large");
     DeviceGuard g(c->device);
     Weight *w = nullptr;
-    int32_t rc = weight_alloc(c, qt, (int64_t)m, (int64_t)k, 0, 1.0f, &w);
+    bool waited = false;
+    int32_t rc = weight_alloc(c, qt, (int64_t)m, (int64_t)k, 0, 1.0f, &w, &waited);
     if (rc) return rc;
-    rc = weight_fill(c, w, wb, nullptr, false);
+    rc = weight_fill(c, w, wb, nullptr, false, waited);
     if (!rc) rc = matmul_host_impl(c, w, input, (int)n, output, true, nullptr, 0);
     weight_destroy(w);
     return rc;
@@ -994,9 +1103,10 @@ static int32_t gemm_kq_host(gllmk_ctx ctx, int32_t qt, const char *what, const v
     if (m > 0x7fffffffu) return fail(c, GLLMK_STATUS_INVALID_ARG, "m too large");
     DeviceGuard g(c->device);
     Weight *w = nullptr;
-    int32_t rc = weight_alloc(c, qt, (int64_t)n, (int64_t)k, 0, 1.0f, &w);
+    bool waited = false;
+    int32_t rc = weight_alloc(c, qt, (int64_t)n, (int64_t)k, 0, 1.0f, &w, &waited);
     if (rc) return rc;
-    rc = weight_fill(c, w, weight, nullptr, false);
+    rc = weight_fill(c, w, weight, nullptr, false, waited);
     if (!rc) rc = matmul_host_impl(c, w, input, (int)m, output, false, scales, n_scales);
     weight_destroy(w);
     return rc;

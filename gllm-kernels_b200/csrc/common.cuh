@@ -64,7 +64,8 @@ struct Weight {
     int64_t nb8 = 0;  // Q8_0: groups of 8 blocks per row
     float global_scale = 1.0f;
     int device = 0;
-    void *qs = nullptr;   // Q4_K / Q8_0 quant plane, FP4 data plane
+    void *qs = nullptr;   // Q4_K / Q8_0 quant plane, FP4 data plane; start of the weight's one allocation
+    size_t alloc_bytes = 0;
     void *aux = nullptr;  // Q4_K headers, Q8_0 scales, FP4 scale-factor plane
     size_t qs_bytes = 0, aux_bytes = 0;
     uint64_t ref_bytes = 0;
@@ -93,6 +94,8 @@ struct Ctx {
     void *dev_io = nullptr;
     size_t dev_io_bytes = 0;
     cudaStream_t stream = nullptr;  // the context's own stream for host-pointer entry points
+    void *host_word = nullptr;      // page-locked word a kernel leaves a result for the host in, and the event that says so
+    cudaEvent_t host_word_ready = nullptr;
     // gllmk_matmul_host_batch: a second stream for the host <-> device copies (they run beside the products), events
     // for the hand-overs, and the instantiated graph of the last argument list that was seen twice
     cudaStream_t copy_stream = nullptr;
@@ -127,17 +130,19 @@ int32_t ensure_act(Ctx *c, size_t bytes);
 int32_t ensure_cnt(Ctx *c, size_t bytes);
 int32_t ensure_pin(Ctx *c, size_t bytes);
 int32_t ensure_dev_io(Ctx *c, size_t bytes);
+int32_t ensure_host_word(Ctx *c);
 
 // Makes the context's device current for the duration of an entry point and restores the caller's.
 struct DeviceGuard {
     int prev = -1;
+    int dev_;
     bool ok = true;
-    explicit DeviceGuard(int dev) {
+    explicit DeviceGuard(int dev) : dev_(dev) {
         if (cudaGetDevice(&prev) != cudaSuccess) { ok = false; (void)cudaGetLastError(); return; }
         if (prev != dev && cudaSetDevice(dev) != cudaSuccess) { ok = false; (void)cudaGetLastError(); }
     }
     ~DeviceGuard() {
-        if (ok && prev >= 0) cudaSetDevice(prev);
+        if (ok && prev >= 0 && prev != dev_) cudaSetDevice(prev);
     }
 };
 
@@ -146,6 +151,23 @@ struct DeviceGuard {
         cudaError_t e__ = (call);                                    \
         if (e__ != cudaSuccess) return cuda_fail((c), e__, #call);   \
     } while (0)
+
+// Programmatic launch: the kernel starts as soon as every block of the kernel in front has issued
+// griddepcontrol.launch_dependents (or ended), and orders what it reads of it with griddepcontrol.wait.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_after(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
 
 // ---- repack.cu ----
 int32_t repack_upload(Ctx *c, Weight *w, const void *blocks_dev, const void *scales_dev, cudaStream_t s);
@@ -201,6 +223,19 @@ int32_t raw_dequant(Ctx *c, int32_t qt, const uint8_t *w, int64_t n, int64_t nb,
 int32_t raw_gemv_launch(Ctx *c, const Weight *w, const float *x, int64_t xst, int64_t xsk, int m, float *y, int64_t yst,
                         int64_t ysr, const float *row_scales, int64_t n_row_scales, cudaStream_t s);
 // ---- quantize.cu ----
+// Largest magnitude of a tensor, in the context's 16 KB of small device scratch (ints behind the status word: 64 .. 127 and
+// the block maxima from 128 on; the expert counts of moe.cu share the area, calls on a context do not overlap)
+constexpr int AMAX_PARTS = 592;  // blocks, four per SM
+struct AmaxOut {
+    float amax, global;  // the maximum; amax / (6 * 448), 1 for an all-zero tensor (NVFP4's global scale)
+    float scale;         // amax / 127 as the W8A8 quantizer wrote it
+    int arrived;         // zero between launches
+    float pad[60];
+    float part[AMAX_PARTS];
+};
+inline AmaxOut *amax_out(const Ctx *c) { return reinterpret_cast<AmaxOut *>(c->status_dev + 64); }
+// rows x k elements, ld apart; host_global (page-locked) may be nullptr.  The kernel issues griddepcontrol.launch_dependents.
+int32_t amax_launch(Ctx *c, const float *x, int64_t rows, int64_t k, int64_t ld, float *host_global, cudaStream_t s);
 int32_t quantize_launch(Ctx *c, int32_t qt, const float *x, int64_t rows, int64_t k, int mx_block, void *blocks,
                         void *scales, float *global_scale, cudaStream_t s);
 

@@ -481,54 +481,10 @@ int32_t i8_weight_fill(Ctx *c, Weight *w, const int8_t *b_dev, int layout, cudaS
 // quantize_from_fp32 / QuantFormat::Int8PerTensor (src/compiler/quant_convert.rs:17-20,165-177): scale = max|x| / 127,
 // q = (x / scale).round().clamp(-128, 127) as i8 (round half away from zero; NaN, i.e. 0 / 0 for an all-zero tensor, -> 0).
 //
-// Two passes, both bound by reading x (the second finds it in L2 up to ~100 MB): block maxima, then every block of the
-// second pass reduces the (at most AQ_PARTS) block maxima itself, under its own loads of x, so there is no atomic, no
-// cleared word and no launch in between.  x [2048, 4096] from a cold cache: 8 + 16 us (4-byte loads, an atomic maximum and a
-// byte image that a third pass turned into tile images: 24 + 41 + 9 us).
-constexpr int AQ_PARTS = 592;      // blocks of the first pass: four per SM
-constexpr int AQ_SCALE_OFF = 72;   // words of the context's small device scratch (behind its status word): scale, maximum
-constexpr int AQ_PART_OFF = 128;   // and the block maxima
-constexpr int AQ_ROWS = 8;         // rows (16-byte loads in flight) per thread of the second pass
-constexpr int AQ_SEG = 4096;       // elements a block takes at a time: four 16-byte loads per thread in flight
-
-__device__ __forceinline__ float max_abs4(float a, float4 v) {
-    // f32::max semantics: a NaN operand is ignored
-    return fmaxf(fmaxf(a, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
-}
-__global__ void __launch_bounds__(256) act_amax_kernel(const float *__restrict__ x, int64_t rows, int64_t k, int64_t ld, int vec,
-                                                       float *__restrict__ partial) {
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    __shared__ float red[8];
-    const int64_t segs = (k + AQ_SEG - 1) / AQ_SEG, units = rows * segs;
-    float a = 0.0f;
-    for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
-        const int64_t r = u / segs, c0 = (u - r * segs) * AQ_SEG;
-        const float *src = x + r * ld + c0;
-        const int n = (int)(k - c0 < AQ_SEG ? k - c0 : AQ_SEG);
-        if (vec) {
-            float4 v[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int c = 4 * ((int)threadIdx.x + 256 * i);
-                v[i] = c < n ? __ldg(reinterpret_cast<const float4 *>(src + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) a = max_abs4(a, v[i]);
-        } else {
-#pragma unroll 8
-            for (int c = threadIdx.x; c < n; c += 256) a = fmaxf(a, fabsf(src[c]));
-        }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int i = 1; i < 8; i++) a = fmaxf(a, red[i]);
-        partial[blockIdx.x] = a;
-    }
-}
+// Two passes, both bound by reading x (the second finds it in L2 up to ~100 MB): the maximum (quantize.cu), then this kernel,
+// whose loads of x run before it waits for the first.  x [2048, 4096] from a cold cache: 8 + 16 us (4-byte loads, an atomic
+// maximum and a byte image that a third pass turned into tile images: 24 + 41 + 9 us).
+constexpr int AQ_ROWS = 8;  // rows (16-byte loads in flight) per thread
 
 // IMG: the quantized activations (as q + 128) go straight into the tile images the integer GEMM copies (128 tokens x 128 k,
 // swizzled); otherwise to q [rows, ldq].  A warp takes 128 k of a row (16 bytes in, 4 bytes out per lane: whole lines both
@@ -537,9 +493,8 @@ __global__ void __launch_bounds__(256) act_amax_kernel(const float *__restrict__
 template <bool IMG>
 __global__ void __launch_bounds__(256) act_quant_i8_kernel(const float *__restrict__ x, int64_t rows, int64_t k, int64_t ld, int vec,
                                                            uint8_t *__restrict__ q, int64_t ldq, int qvec, int offset,
-                                                           const float *__restrict__ partial, int nparts, float *scale_out) {
+                                                           const AmaxOut *amax, float *scale_out) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    __shared__ float red[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t k0 = (int64_t)blockIdx.x * 128 + 4 * lane;
     float4 v[AQ_ROWS];
@@ -558,19 +513,11 @@ __global__ void __launch_bounds__(256) act_quant_i8_kernel(const float *__restri
             }
         }
     }
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the block maxima are complete from here on
-    float a = 0.0f;
-    for (int i = threadIdx.x; i < nparts; i += 256) a = fmaxf(a, __ldcg(partial + i));
-#pragma unroll
-    for (int o = 16; o; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
-    if (lane == 0) red[warp] = a;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 8; i++) a = fmaxf(a, red[i]);
-    const float scale = __fdiv_rn(a, 127.0f);
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the maximum is complete from here on
+    const float a = __ldcg(&amax->amax), scale = __fdiv_rn(a, 127.0f);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         scale_out[0] = scale;
-        scale_out[1] = a;
+        if (!IMG) scale_out[1] = a;
     }
     // f / scale, correctly rounded: one reciprocal for all elements and two of Markstein's corrections (the first makes the
     // quotient faithful, the second exact); scales so small or large that a step could leave the normal range divide
@@ -607,43 +554,22 @@ __global__ void __launch_bounds__(256) act_quant_i8_kernel(const float *__restri
     }
 }
 
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_after(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
-    // programmatic launch: starts as soon as every block of the kernel in front has issued griddepcontrol.launch_dependents
-    // (and orders its own reads after it with griddepcontrol.wait)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
-}
-
 // img: q is the tile images of the integer GEMM (ldq unused), otherwise [rows, ldq] bytes
 static int32_t act_quant(Ctx *c, const float *x, int64_t rows, int64_t k, int64_t ld, uint8_t *q, int64_t ldq, int offset, bool img,
                          float *scale_dev, cudaStream_t s) {
-    float *partial = reinterpret_cast<float *>(c->status_dev) + AQ_PART_OFF;
     const int vec = (((uintptr_t)x & 15) == 0 && ld % 4 == 0 && k % 4 == 0) ? 1 : 0;
     const int qvec = (((uintptr_t)q & 3) == 0 && ldq % 4 == 0) ? 1 : 0;
-    // contiguous rows are one long row to the maximum
-    const int64_t ar = ld == k ? 1 : rows, ak = ld == k ? rows * k : k;
-    const int64_t units = ar * ((ak + AQ_SEG - 1) / AQ_SEG);
-    const int parts = (int)(units < AQ_PARTS ? units : AQ_PARTS);
-    act_amax_kernel<<<(unsigned)parts, 256, 0, s>>>(x, ar, ak, ld, vec, partial);
-    GK_CUDA(c, cudaGetLastError());
+    const int32_t rc = amax_launch(c, x, rows, k, ld, nullptr, s);
+    if (rc) return rc;
+    const AmaxOut *amax = amax_out(c);
     // row groups beyond the grid's y limit: launches of their own (each writes the same scale)
     const int64_t step = (int64_t)65534 * 8 * AQ_ROWS;  // a multiple of the 128 rows of an image
     for (int64_t r0 = 0; r0 < rows; r0 += step) {
         const int64_t nr = rows - r0 < step ? rows - r0 : step;
         const dim3 grid((unsigned)((k + 127) / 128), (unsigned)((nr + 8 * AQ_ROWS - 1) / (8 * AQ_ROWS)));
         uint8_t *dst = img ? q + (size_t)(r0 >> 7) * ((size_t)(k + 127) / 128) * I8_TILE : q + r0 * ldq;
-        GK_CUDA(c, img ? launch_after(act_quant_i8_kernel<true>, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, partial, parts, scale_dev)
-                       : launch_after(act_quant_i8_kernel<false>, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, partial, parts, scale_dev));
+        GK_CUDA(c, img ? launch_after(act_quant_i8_kernel<true>, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, amax, scale_dev)
+                       : launch_after(act_quant_i8_kernel<false>, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, amax, scale_dev));
     }
     return GLLMK_STATUS_OK;
 }
@@ -740,7 +666,7 @@ int32_t w8a8_linear_launch(Ctx *c, const Weight *w, const float *x, int64_t ldx,
                            int act, cudaStream_t s) {
     int32_t rc = ensure_act(c, (size_t)i8_act_tiles(m) * (size_t)(w->k_pad / 128) * I8_TILE);
     if (rc) return rc;
-    float *scale = reinterpret_cast<float *>(c->status_dev) + AQ_SCALE_OFF;
+    float *scale = &amax_out(c)->scale;
     rc = act_quant(c, x, m, w->k, ldx, static_cast<uint8_t *>(c->act), 0, 128, true, scale, s);
     if (rc) return rc;
     I8Params p{};

@@ -24,6 +24,51 @@ __device__ __forceinline__ uint32_t nearest_e2m1(float v) {
     return (uint32_t)best | ((v < 0.0f) ? 8u : 0u);
 }
 
+// Eight values -> one word of E2M1 codes (nearest_e2m1 of each; element 0 in the low nibble) by the hardware conversion, which
+// rounds to nearest with ties to the even code as well.  It keeps the sign of a zero, which is taken off again.
+__device__ __forceinline__ uint32_t e2m1x8(const float (&v)[8]) {
+    uint32_t w;
+    asm("{\n.reg .b8 a, b, c, d;\n"
+        "cvt.rn.satfinite.e2m1x2.f32 a, %2, %1;\ncvt.rn.satfinite.e2m1x2.f32 b, %4, %3;\n"
+        "cvt.rn.satfinite.e2m1x2.f32 c, %6, %5;\ncvt.rn.satfinite.e2m1x2.f32 d, %8, %7;\n"
+        "mov.b32 %0, {a, b, c, d};\n}\n"
+        : "=r"(w)
+        : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
+    const uint32_t nonzero = ((w & 0x77777777u) + 0x77777777u) & 0x88888888u;  // bit 3 of every nibble whose magnitude is not 0
+    return w & (0x77777777u | nonzero);
+}
+// largest magnitude the conversion above is used for (beyond it, and for NaN, nearest_e2m1 decides value by value: the scale
+// was clamped, or the input is not finite)
+constexpr float E2M1_FAST = 1024.0f;
+__device__ __forceinline__ bool all_below(const float (&v)[8], float lim) {
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 8; i++) ok = ok && fabsf(v[i]) < lim;  // false for NaN
+    return ok;
+}
+__device__ __noinline__ uint32_t e2m1x8_slow(const float (&v)[8]) {
+    uint32_t w = 0;
+    for (int i = 0; i < 8; i++) w |= nearest_e2m1(v[i]) << (4 * i);
+    return w;
+}
+// eight consecutive floats; vec = the address is 16-byte aligned
+__device__ __forceinline__ void load8(const float *x, int vec, float (&v)[8]) {
+    if (vec) {
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(x)), b = __ldg(reinterpret_cast<const float4 *>(x) + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = __ldg(x + i);
+    }
+}
+__device__ __forceinline__ float max_abs8(const float (&v)[8]) {
+    float a = fabsf(v[0]);
+#pragma unroll
+    for (int i = 1; i < 8; i++) a = fmaxf(a, fabsf(v[i]));
+    return a;
+}
+
 // f32_to_e4m3, src/compiler/codegen/vm/numerical_sim.rs:2751-2808, for v >= 0
 __device__ __forceinline__ uint32_t f32_to_ue4m3(float v) {
     if (v != v) return 0x7Fu;
@@ -120,75 +165,169 @@ __global__ void __launch_bounds__(256) quantize_q80_kernel(const float *__restri
     b[2 + lane] = (uint8_t)(int8_t)q;
 }
 
-// ---- MXFP4 (block 32): one warp per block, split output (16 nibble bytes + 1 E8M0 byte) ----
-__global__ void __launch_bounds__(256) quantize_mxfp4_kernel(const float *__restrict__ x, uint8_t *__restrict__ blocks,
-                                                              uint8_t *__restrict__ scales, size_t nblocks) {
-    const size_t blk = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (blk >= nblocks) return;
-    const float v = x[blk * 32 + lane];
-    float amax = fabsf(v);
+// The two FP4 encoders are bound by reading x once.  A lane takes eight consecutive elements (two 16-byte loads, one 4-byte
+// store of codes), two such units in flight per thread; the block's maximum is a few shuffles.  x [2048, 4096], NVFP4, from a
+// cold cache: 12 us (34 with 8-byte loads, 1-byte stores, a search of the eight magnitudes and an IEEE division per element).
+constexpr int QF_UNITS = 2;
+
+// ---- MXFP4 (block 32 = 4 lanes), split output (16 nibble bytes + 1 E8M0 byte) ----
+__global__ void __launch_bounds__(256) quantize_mxfp4_kernel(const float *__restrict__ x, int vec, uint32_t *__restrict__ blocks,
+                                                              uint8_t *__restrict__ scales, size_t units) {
+    const size_t u0 = (size_t)blockIdx.x * (256 * QF_UNITS) + threadIdx.x;
+    float v[QF_UNITS][8];
 #pragma unroll
-    for (int d = 16; d; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
-    int byte = 127;
-    if (amax > 0.0f) {
-        int p;
-        const float f = frexpf(amax, &p);  // smallest e with 6 * 2^e >= amax
-        const int e = (f <= 0.75f) ? p - 3 : p - 2;
-        byte = clampi(e + 127, 1, 254);
+    for (int j = 0; j < QF_UNITS; j++) {
+        const size_t u = u0 + 256 * j;
+        if (u < units) load8(x + 8 * u, vec, v[j]);
+        else
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[j][i] = 0.0f;
     }
-    const float inv = ldexpf(1.0f, 127 - byte);
-    const uint32_t code = nearest_e2m1(v * inv);
-    const uint32_t hi = __shfl_down_sync(0xffffffffu, code, 1);
-    if ((lane & 1) == 0) blocks[blk * 16 + (lane >> 1)] = (uint8_t)(code | (hi << 4));
-    if (lane == 0) scales[blk] = (uint8_t)byte;
+#pragma unroll
+    for (int j = 0; j < QF_UNITS; j++) {
+        const size_t u = u0 + 256 * j;
+        float amax = max_abs8(v[j]);
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        int byte = 127;
+        if (amax > 0.0f) {
+            int p;
+            const float f = frexpf(amax, &p);  // smallest e with 6 * 2^e >= amax
+            const int e = (f <= 0.75f) ? p - 3 : p - 2;
+            byte = clampi(e + 127, 1, 254);
+        }
+        // 2^(127 - byte), exactly (byte 254: 2^-127, a subnormal)
+        const float inv = __int_as_float(byte == 254 ? 0x00400000 : (254 - byte) << 23);
+        float q[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) q[i] = v[j][i] * inv;
+        const uint32_t w = all_below(q, E2M1_FAST) ? e2m1x8(q) : e2m1x8_slow(q);
+        if (u < units) {
+            blocks[u] = w;
+            if ((u & 3) == 0) scales[u >> 2] = (uint8_t)byte;
+        }
+    }
 }
 
-// ---- NVFP4 (block 64 = 4 x 16): one warp per block, lane handles elements 2*lane, 2*lane+1 ----
-__global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const float *__restrict__ x, uint8_t *__restrict__ out,
-                                                              const float *__restrict__ global_ptr, size_t nblocks) {
-    const size_t blk = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (blk >= nblocks) return;
-    const float global = *global_ptr;
-    const float2 v = *reinterpret_cast<const float2 *>(x + blk * 64 + 2 * lane);
-    float amax = fmaxf(fabsf(v.x), fabsf(v.y));
+// ---- NVFP4 (block 64 = 4 x 16 elements, 8 lanes): 4 UE4M3 bytes, 32 code bytes; global from device memory or by value ----
+__global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const float *__restrict__ x, int vec, uint8_t *__restrict__ out,
+                                                              const float *__restrict__ global_ptr, float global, size_t units) {
+    const size_t u0 = (size_t)blockIdx.x * (256 * QF_UNITS) + threadIdx.x;
+    float v[QF_UNITS][8];
 #pragma unroll
-    for (int d = 4; d; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));  // 8 lanes = 16 el
-    const uint32_t sb = f32_to_ue4m3(amax / (6.0f * global)) & 0x7Fu;
-    const float s = global * e4m3_to_f32(sb);
-    uint32_t lo = 0, hi = 0;
-    if (s > 0.0f) {
-        lo = nearest_e2m1(v.x / s);
-        hi = nearest_e2m1(v.y / s);
+    for (int j = 0; j < QF_UNITS; j++) {
+        const size_t u = u0 + 256 * j;
+        if (u < units) load8(x + 8 * u, vec, v[j]);
+        else
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[j][i] = 0.0f;
     }
-    uint8_t *b = out + blk * 36;
-    if ((lane & 7) == 0) b[lane >> 3] = (uint8_t)sb;
-    b[4 + lane] = (uint8_t)(lo | (hi << 4));
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the global scale is complete from here on
+    if (global_ptr) global = __ldcg(global_ptr);
+#pragma unroll
+    for (int j = 0; j < QF_UNITS; j++) {
+        const size_t u = u0 + 256 * j;
+        float amax = max_abs8(v[j]);
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));  // 2 lanes = 16 elements
+        const uint32_t sb = f32_to_ue4m3(amax / (6.0f * global)) & 0x7Fu;
+        const float s = global * e4m3_to_f32(sb);
+        uint32_t w = 0;
+        if (s > 0.0f) {
+            // v / s, correctly rounded: one reciprocal per lane and two of Markstein's corrections per element (the first makes
+            // the quotient faithful, the second exact) where no step can leave the normal range
+            float q[8];
+            const bool fast = s > 1e-30f && s < 1e30f;
+            const float y = fast ? __frcp_rn(s) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                float d = v[j][i] * y;
+                d = fmaf(fmaf(-d, s, v[j][i]), y, d);
+                q[i] = fmaf(fmaf(-d, s, v[j][i]), y, d);
+            }
+            if (fast && all_below(q, E2M1_FAST)) {
+                w = e2m1x8(q);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; i++) q[i] = v[j][i] / s;
+                w = e2m1x8_slow(q);
+            }
+        }
+        if (u < units) {
+            uint8_t *b = out + (u >> 3) * 36;
+            *reinterpret_cast<uint32_t *>(b + 4 + 4 * (u & 7)) = w;
+            if ((u & 1) == 0) b[(u & 7) >> 1] = (uint8_t)sb;
+        }
+    }
 }
 
-// amax over a tensor -> global = amax / (6 * 448), 1 when all zero.  Two small passes.
-__global__ void __launch_bounds__(256) amax_partial_kernel(const float *__restrict__ x, size_t count,
-                                                            float *__restrict__ partial) {
+// ---- largest magnitude of a tensor (f32::max semantics: NaN is ignored) ---------------------------------------------
+// Bound by reading x: 16-byte loads, eight in flight per thread; block maxima in the context's small device scratch, and the
+// block that finishes last reduces them and writes what the next kernel needs, so no other launch lies in between.
+// x [2048, 4096] from a cold cache: 11 us (25 us with 4-byte loads and an atomic maximum, 32 us with 4-byte loads and a
+// second launch; without the last block's reduction 8 us, but then every block of the next kernel has to do it).
+constexpr int AMAX_SEG = 8192;  // elements a block takes at a time
+__global__ void __launch_bounds__(256) amax_kernel(const float *__restrict__ x, int64_t rows, int64_t k, int64_t ld, int vec, AmaxOut *out,
+                                                   float *host_global) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     __shared__ float red[8];
+    __shared__ int last_s;
+    const int64_t segs = (k + AMAX_SEG - 1) / AMAX_SEG, units = rows * segs;
     float a = 0.0f;
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < count; i += (size_t)gridDim.x * 256)
-        a = fmaxf(a, fabsf(x[i]));
+    for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
+        const int64_t r = u / segs, c0 = (u - r * segs) * AMAX_SEG;
+        const float *src = x + r * ld + c0;
+        const int n = (int)(k - c0 < AMAX_SEG ? k - c0 : AMAX_SEG);
+        if (vec) {
+            float4 v[8];
 #pragma unroll
-    for (int d = 16; d; d >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, d));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
-    __syncthreads();
+            for (int i = 0; i < 8; i++) {
+                const int c = 4 * ((int)threadIdx.x + 256 * i);
+                v[i] = c < n ? __ldg(reinterpret_cast<const float4 *>(src + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) a = fmaxf(fmaxf(a, fmaxf(fabsf(v[i].x), fabsf(v[i].y))), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));
+        } else {
+#pragma unroll 8
+            for (int c = threadIdx.x; c < n; c += 256) a = fmaxf(a, fabsf(src[c]));
+        }
+    }
+    const auto block_max = [&]() {  // valid in thread 0
+#pragma unroll
+        for (int o = 16; o; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 8; i++) a = fmaxf(a, red[i]);
+    };
+    block_max();
     if (threadIdx.x == 0) {
-        for (int i = 1; i < 8; i++) a = fmaxf(a, red[i]);
-        partial[blockIdx.x] = a;
+        __stcg(out->part + blockIdx.x, a);
+        __threadfence();
+        last_s = atomicAdd(&out->arrived, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    a = 0.0f;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += 256) a = fmaxf(a, __ldcg(out->part + i));
+    __syncthreads();
+    block_max();
+    if (threadIdx.x == 0) {
+        const float g = (a > 0.0f) ? a / (6.0f * 448.0f) : 1.0f;  // NVFP4's global scale, 1 when all zero
+        out->arrived = 0;  // ready for the next launch
+        out->amax = a;
+        out->global = g;
+        if (host_global) *reinterpret_cast<volatile float *>(host_global) = g;  // page-locked host memory
     }
 }
-__global__ void amax_final_kernel(const float *__restrict__ partial, int n, float *__restrict__ global_out) {
-    float a = 0.0f;
-    for (int i = threadIdx.x; i < n; i += 32) a = fmaxf(a, partial[i]);
-#pragma unroll
-    for (int d = 16; d; d >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, d));
-    if (threadIdx.x == 0) *global_out = (a > 0.0f) ? a / (6.0f * 448.0f) : 1.0f;
+
+int32_t amax_launch(Ctx *c, const float *x, int64_t rows, int64_t k, int64_t ld, float *host_global, cudaStream_t s) {
+    const int vec = (((uintptr_t)x & 15) == 0 && ld % 4 == 0 && k % 4 == 0) ? 1 : 0;
+    if (ld == k) k *= rows, rows = 1;  // contiguous rows are one long row
+    const int64_t units = rows * ((k + AMAX_SEG - 1) / AMAX_SEG);
+    amax_kernel<<<(unsigned)(units < AMAX_PARTS ? units : AMAX_PARTS), 256, 0, s>>>(x, rows, k, ld, vec, amax_out(c), host_global);
+    GK_CUDA(c, cudaGetLastError());
+    return GLLMK_STATUS_OK;
 }
 
 int32_t quantize_launch(Ctx *c, int32_t qt, const float *x, int64_t rows, int64_t k, int mx_block, void *blocks,
@@ -202,24 +341,29 @@ int32_t quantize_launch(Ctx *c, int32_t qt, const float *x, int64_t rows, int64_
         quantize_q80_kernel<<<(unsigned)((nb + 7) / 8), 256, 0, s>>>(x, (uint8_t *)blocks, nb);
     } else if (qt == GLLMK_QUANT_MXFP4) {
         if (mx_block != 32) return fail(c, GLLMK_STATUS_UNSUPPORTED, "quantize: MXFP4 block_size %d (only 32)", mx_block);
-        const size_t nb = count / 32;
-        quantize_mxfp4_kernel<<<(unsigned)((nb + 7) / 8), 256, 0, s>>>(x, (uint8_t *)blocks, (uint8_t *)scales, nb);
+        const size_t units = count / 8;
+        quantize_mxfp4_kernel<<<(unsigned)((units + 256 * QF_UNITS - 1) / (256 * QF_UNITS)), 256, 0, s>>>(
+            x, ((uintptr_t)x & 15) == 0, (uint32_t *)blocks, (uint8_t *)scales, units);
     } else if (qt == GLLMK_QUANT_NVFP4) {
-        // scratch behind the status word (16 KiB block owned by the context): global scale + partial maxima
-        float *gdev = reinterpret_cast<float *>(c->status_dev) + 64;
-        float *partial = gdev + 64;
-        if (*global_scale > 0.0f) {
-            GK_CUDA(c, cudaMemcpyAsync(gdev, global_scale, sizeof(float), cudaMemcpyHostToDevice, s));
-        } else {
-            const int nblk = (int)((count + 256 * 64 - 1) / (256 * 64) < 1024 ? (count + 256 * 64 - 1) / (256 * 64) : 1024);
-            amax_partial_kernel<<<nblk, 256, 0, s>>>(x, count, partial);
-            amax_final_kernel<<<1, 32, 0, s>>>(partial, nblk, gdev);
+        const bool given = *global_scale > 0.0f;
+        if (!given) {
+            // the scale goes to the host as soon as the first pass has it; the encoder runs under the host's wait and the
+            // caller's next steps
+            int32_t rc = ensure_host_word(c);
+            if (!rc) rc = amax_launch(c, x, 1, (int64_t)count, (int64_t)count, static_cast<float *>(c->host_word), s);
+            if (rc) return rc;
+            GK_CUDA(c, cudaEventRecord(c->host_word_ready, s));
         }
-        const size_t nb = count / 64;
-        quantize_nvfp4_kernel<<<(unsigned)((nb + 7) / 8), 256, 0, s>>>(x, (uint8_t *)blocks, gdev, nb);
-        if (!(*global_scale > 0.0f)) {
-            GK_CUDA(c, cudaMemcpyAsync(global_scale, gdev, sizeof(float), cudaMemcpyDeviceToHost, s));
-            GK_CUDA(c, cudaStreamSynchronize(s));
+        const size_t units = count / 8;
+        const unsigned grid = (unsigned)((units + 256 * QF_UNITS - 1) / (256 * QF_UNITS));
+        const int vec = ((uintptr_t)x & 15) == 0;
+        uint8_t *out = static_cast<uint8_t *>(blocks);
+        if (given) quantize_nvfp4_kernel<<<grid, 256, 0, s>>>(x, vec, out, nullptr, *global_scale, units);
+        else GK_CUDA(c, launch_after(quantize_nvfp4_kernel, dim3(grid), 256, 0, s, x, vec, out, &amax_out(c)->global, 0.0f, units));
+        GK_CUDA(c, cudaGetLastError());
+        if (!given) {
+            GK_CUDA(c, cudaEventSynchronize(c->host_word_ready));
+            *global_scale = *static_cast<volatile float *>(c->host_word);
         }
     } else {
         return fail(c, GLLMK_STATUS_UNSUPPORTED, "quantize: unknown quant type %d", qt);

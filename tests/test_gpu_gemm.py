@@ -430,3 +430,36 @@ def test_ffn_prefill_swiglu(gk, K, oracle, fmt, d, f, m, x_bf16):
     assert e.value.status == gk.Status.INVALID_ARG
     w_gu.free()
     w_dn.free()
+
+
+@pytest.mark.parametrize("ms", [(300, 300, 300), (257, 300, 511, 129), (1, 40, 2000)])
+def test_fp4_activations_uploaded_per_call_reuse_freed_buffers(gk, K, ms):
+    """Activation matrices come and go like weights while earlier products may still be reading theirs: a freed buffer is
+    taken again only after the device has been waited for.  Products launched back to back on two streams, each matrix freed
+    right after its launch, must equal the same products run one at a time with every matrix kept alive."""
+    import torch
+    n, k = 384, 1024
+    qt = gk.QuantType.nvfp4()
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    wb, wg = K.quantize(qt, torch.randn((n, k), device="cuda", generator=gen))
+    w = K.upload(qt, n, k, wb, None, wg)
+    xs = [torch.randn((m, k), device="cuda", generator=gen) for m in ms for _ in range(3)]
+    ref, keep = [], []
+    for x in xs:
+        b, g = K.quantize(qt, x)
+        keep.append(K.upload(qt, x.shape[0], k, b, None, g))
+        ref.append(K.gemm_fp4(w, keep[-1]))
+        torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    got = []
+    for i, x in enumerate(xs):
+        with torch.cuda.stream(streams[i % 2]):
+            b, g = K.quantize(qt, x)
+            X = K.upload(qt, x.shape[0], k, b, None, g)
+            got.append(K.gemm_fp4(w, X))
+            X.free()
+    torch.cuda.synchronize()
+    assert K.status() == 0
+    for a, b in zip(got, ref):
+        assert torch.equal(a, b)

@@ -539,3 +539,30 @@ def test_matmul_host_batch_equals_one_call_per_product(gk, K, oracle, torch):
     assert e.value.status == gk.Status.INVALID_ARG
     for w in ws:
         w.free()
+
+
+@pytest.mark.parametrize("fmt,n,k,offset,global_scale", [("nvfp4", 3, 64, 0, 0.0), ("nvfp4", 1, 64 * 129, 1, 0.0), ("nvfp4", 7, 4096, 0, 1e-6), ("nvfp4", 33, 640, 2, 1e-3),
+                                                         ("mxfp4", 1, 32, 0, 0.0), ("mxfp4", 5, 32 * 257, 3, 0.0), ("mxfp4", 64, 2048, 0, 0.0)])
+def test_fp4_quantizers_ties_clamps_and_alignment(gk, K, oracle, torch, fmt, n, k, offset, global_scale):
+    """The FP4 encoders byte for byte against the oracle where they could differ: values on the ties between two E2M1 codes,
+    negative values that round to zero, a given global scale so small that block scales clamp and codes saturate, tensors that
+    end inside a thread's unit, an input that is not 16-byte aligned."""
+    rng = np.random.default_rng(n * k + offset)
+    W = rng.standard_normal((n, k)).astype(np.float32)
+    ties = np.array([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0, 6.0, -0.25, -0.75, -1.25, -1.75, -2.5, -3.5, -5.0, -0.1], np.float32)
+    W[0, :16] = ties                      # block maximum 6: scale 1, every tie exact
+    W[-1, -16:] = ties * np.float32(2.0 ** -9)
+    W[0, 16:32] = -1e-30
+    buf = torch.zeros(n * k + 4, device="cuda")
+    buf[offset:offset + n * k] = torch.from_numpy(W).cuda().reshape(-1)
+    xd = buf[offset:offset + n * k].view(n, k)
+    if fmt == "mxfp4":
+        b, s = K.quantize(qt_of(gk, fmt), xd)
+        rb, rs = oracle.quantize_mxfp4(W)
+        assert np.array_equal(b.cpu().numpy(), rb) and np.array_equal(s.cpu().numpy(), rs)
+    else:
+        global_scale = float(np.float32(global_scale))
+        b, g = K.quantize(qt_of(gk, fmt), xd, global_scale=global_scale)
+        rb, rg = oracle.quantize_nvfp4(W, global_scale) if global_scale else oracle.quantize_nvfp4(W)
+        assert g == pytest.approx(rg, rel=0, abs=0)
+        assert np.array_equal(b.cpu().numpy(), rb)
