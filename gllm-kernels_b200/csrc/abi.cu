@@ -55,7 +55,7 @@ int32_t ensure_cnt(Ctx *c, size_t bytes) {
 }
 int32_t ensure_pin(Ctx *c, size_t bytes) { return grow(c, &c->pin, &c->pin_bytes, bytes, true); }
 int32_t ensure_host_word(Ctx *c) {
-    if (!c->host_word) GK_CUDA(c, cudaMallocHost(&c->host_word, 64));
+    if (!c->host_word) GK_CUDA(c, cudaMallocHost(&c->host_word, 8192));
     if (!c->host_word_ready) GK_CUDA(c, cudaEventCreateWithFlags(&c->host_word_ready, cudaEventDisableTiming));
     return GLLMK_STATUS_OK;
 }

@@ -94,8 +94,8 @@ struct Ctx {
     void *dev_io = nullptr;
     size_t dev_io_bytes = 0;
     cudaStream_t stream = nullptr;  // the context's own stream for host-pointer entry points
-    void *host_word = nullptr;      // page-locked word a kernel leaves a result for the host in, and the event that says so
-    cudaEvent_t host_word_ready = nullptr;
+    void *host_word = nullptr;      // 8 KB of page-locked memory kernels leave small results for the host in (a scale, 1025 row offsets)
+    cudaEvent_t host_word_ready = nullptr;  // recorded behind the kernel that wrote it
     // gllmk_matmul_host_batch: a second stream for the host <-> device copies (they run beside the products), events
     // for the hand-overs, and the instantiated graph of the last argument list that was seen twice
     cudaStream_t copy_stream = nullptr;
@@ -224,7 +224,7 @@ int32_t raw_gemv_launch(Ctx *c, const Weight *w, const float *x, int64_t xst, in
                         int64_t ysr, const float *row_scales, int64_t n_row_scales, cudaStream_t s);
 // ---- quantize.cu ----
 // Largest magnitude of a tensor, in the context's 16 KB of small device scratch (ints behind the status word: 64 .. 127 and
-// the block maxima from 128 on; the expert counts of moe.cu share the area, calls on a context do not overlap)
+// the block maxima from 128 on)
 constexpr int AMAX_PARTS = 592;  // blocks, four per SM
 struct AmaxOut {
     float amax, global;  // the maximum; amax / (6 * 448), 1 for an all-zero tensor (NVFP4's global scale)

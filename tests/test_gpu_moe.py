@@ -101,3 +101,33 @@ def test_moe_argument_checks(gk, K):
     with pytest.raises(gk.GllmkError) as e:
         K.moe_route(r, 4, 2000, 2)
     assert e.value.status == gk.Status.UNSUPPORTED
+
+
+@pytest.mark.parametrize("T,E,top_k,k,H,pad", [(1, 1, 1, 8, 4, 0), (300, 1024, 4, 264, 1028, 0), (5000, 16, 2, 7, 3, 0), (129, 8, 16, 520, 512, 0), (64, 32, 8, 258, 260, 1),
+                                               (1025, 7, 3, 4096, 2048, 4)])
+def test_moe_kernels_edges(gk, K, oracle, T, E, top_k, k, H, pad):
+    """Slot counts around a warp's and a step's share of the routing kernel, expert counts up to its limit, top_k up to every
+    size of the register list, row lengths and leading dimensions of every copy width, more terms than are loaded at once."""
+    import torch
+    rng = np.random.default_rng(T + E + k)
+    probs = rng.random((T, E), dtype=np.float32)
+    routing = K.moe_topk(torch.from_numpy(probs).cuda(), top_k)
+    ref = oracle.scalar_topk(probs, top_k)
+    got = routing.cpu().numpy()
+    assert ((got.view(np.uint32) == ref.view(np.uint32)) | (np.isnan(got) & np.isnan(ref))).all()
+    offs, perm, inv = K.moe_route(routing, T, E, top_k)
+    idx = ref[0].view(np.uint32)
+    order = np.argsort(idx, kind="stable")
+    assert offs == [0] + np.cumsum(np.bincount(idx, minlength=E)).tolist()
+    assert np.array_equal(perm.cpu().numpy(), order)
+    inv_h = np.empty(T * top_k, np.int64)
+    inv_h[order] = np.arange(T * top_k)
+    assert np.array_equal(inv.cpu().numpy(), inv_h)
+    for dt in (torch.float32, torch.bfloat16):
+        wide = torch.randn((T, k + pad), device="cuda").to(dt)
+        assert torch.equal(K.moe_gather(wide[:, :k], perm, top_k), wide[torch.from_numpy(order // top_k).cuda(), :k])
+    rows = torch.randn((T * top_k, H + pad), device="cuda")[:, :H]
+    out = K.moe_weighted_sum(rows, routing, inv, T, top_k).cpu().numpy()
+    want = oracle.scalar_weighted_sum_grouped(np.ascontiguousarray(rows.cpu().numpy()), ref, inv_h, T, top_k)
+    ok = ~np.isnan(want)
+    assert np.array_equal(out.view(np.uint32)[ok], want.view(np.uint32)[ok])
