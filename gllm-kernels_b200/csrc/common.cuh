@@ -117,7 +117,7 @@ struct Ctx {
                                 // 1 when the estimate favours it, 2 always
     int64_t gemm_raw_slots = 0;  // weight-only GEMM: raw super-chunk ring depth (0 = chosen by the shared-memory plan)
     int64_t gemm_pdl = 1;        // weight-only GEMM launched programmatically behind its activation staging kernel
-    int64_t raw_gemv_mma = 1;    // Q6_K products of 2 tokens and more on the tensor-core kernel (0 = dp2a kernel, 2 = also a single token)
+    int64_t raw_gemv_mma = 1;    // Q4_0 / Q5_0 rows of whole 256-element groups: 0 = the dp2a kernel (the other row-major formats have one kernel)
     int64_t gemm_row_tiles = 0;  // weight-only GEMM: row tiles per CTA (0 = estimated, 1, 2)
     int64_t peer_wait_spins = (int64_t)1 << 22;  // probes of another rank's flag before a wait gives up (status 31 / 32)
 };
@@ -222,6 +222,10 @@ int32_t raw_dequant(Ctx *c, int32_t qt, const uint8_t *w, int64_t n, int64_t nb,
                     cudaStream_t s, bool dev_layout);
 int32_t raw_gemv_launch(Ctx *c, const Weight *w, const float *x, int64_t xst, int64_t xsk, int m, float *y, int64_t yst,
                         int64_t ysr, const float *row_scales, int64_t n_row_scales, cudaStream_t s);
+// ---- gemv_raw.cu: the same formats' decode products on the integer tensor core ----
+bool raw_mma_takes(const Ctx *c, const Weight *w);
+int32_t raw_mma_launch(Ctx *c, const Weight *w, const float *x, int64_t xst, int64_t xsk, int m, float *y, int64_t yst, int64_t ysr,
+                       const float *row_scales, int64_t n_row_scales, cudaStream_t s);
 // ---- quantize.cu ----
 // Largest magnitude of a tensor, in the context's 16 KB of small device scratch (ints behind the status word: 64 .. 127 and
 // the block maxima from 128 on)
