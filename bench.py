@@ -1201,8 +1201,8 @@ def run_w8a8_case(args, K, gk, torch, dev, gen):
 
 
 def run_gguf_case(args, K, gk, torch, dev, gen):
-    """Q6_K decode product on its own: W[8192, 28672] (the down projection of config 5), M = --m tokens (1: the dp2a kernel,
-    2 .. 16: the mma.sync kernel), two weight copies in rotation (2 x 193 MB > L2)."""
+    """Q6_K decode product on its own: W[8192, 28672] (the down projection of config 5), M = --m tokens
+    (1 .. 16: raw_mma_gemv_kernel), two weight copies in rotation (2 x 193 MB > L2)."""
     qt = gk.QuantType.q6k()
     n, k = D_MODEL, N_FF
     nblk = n * (k // 256)
@@ -1233,7 +1233,7 @@ def run_gguf_case(args, K, gk, torch, dev, gen):
                       "warmup": max(args.warmup, 3), "ms_per_step": ms, "higher_is_better": True, "data": "synthetic",
                       "config": {"workload": args.case, "n": n, "k": k, "m": m, "l2": "two weight copies in rotation"},
                       "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
-                                   "traffic": None, "peak_kind": kind, "kernel": ("raw_gemv_kernel<Q6_K, 1>" if m == 1 else "q6k_gemv_mma_kernel") + " (+ act_quant_kernel)"},
+                                   "traffic": None, "peak_kind": kind, "kernel": "raw_mma_gemv_kernel<Q6_K> (+ raw_mma_stage_kernel)"},
                       "gpu_launches": args.steps * 2, "status": K.status()}), flush=True)
 
 

@@ -592,11 +592,12 @@ int32_t gllmk_gemm(gllmk_ctx ctx, gllmk_weight wh, const void *a_dev, int32_t a_
     if (w->device != c->device) return fail(c, GLLMK_STATUS_INVALID_ARG, "weight lives on another device");
     DeviceGuard g(c->device);
     // Q6_K, Q5_K and (when a row's blocks come in whole 16-byte aligned groups of eight: k a multiple of 256) Q4_0 / Q5_0 have
-    // a place in the fused-dequant tensor-core GEMM.  On W[8192, 28672] it takes ~100 us up to 128 tokens; Q6_K's batch GEMV
-    // needs 100 us up to 8 tokens and 135 us up to 16, the dp2a kernel of the other three 150 - 170 us for 2 tokens and
-    // 590 us for 16
-    if ((w->qt == GLLMK_QUANT_Q6_K && m > 8) || (w->qt == GLLMK_QUANT_Q5_K && m >= 2) ||
-        ((w->qt == GLLMK_QUANT_Q4_0 || w->qt == GLLMK_QUANT_Q5_0) && w->k % 256 == 0 && m >= 2))
+    // a place in the fused-dequant tensor-core GEMM.  On W[8192, 28672] it takes ~100 us up to 128 tokens; the decode kernel, f32
+    // in and out only, 50 - 72 us up to 8 tokens and 82 - 95 us (Q6_K: 117) up to 16
+    const bool f32 = a_dtype == GLLMK_DTYPE_F32 && y_dtype == GLLMK_DTYPE_F32 && ((uintptr_t)a_dev & 15) == 0 && lda % 4 == 0;
+    if ((w->qt == GLLMK_QUANT_Q6_K && m > 8) ||
+        ((w->qt == GLLMK_QUANT_Q5_K || ((w->qt == GLLMK_QUANT_Q4_0 || w->qt == GLLMK_QUANT_Q5_0) && w->k % 256 == 0)) && m >= 2 &&
+         !(f32 && m <= GLLMK_GEMM_GEMV_MAX_M)))
         return gemm_launch(c, w, a_dev, a_dtype == GLLMK_DTYPE_BF16, lda, m, y_dev, y_dtype == GLLMK_DTYPE_BF16, ldy,
                            static_cast<cudaStream_t>(stream));
     if (raw_format(w->qt)) {

@@ -15,9 +15,15 @@
 // contiguous bytes) through a ring of stages, together with the block's activation slice, which the eight warps share.  The
 // (row group, block) sequence is cut evenly over the resident CTAs and partial sums meet in gemv.cu's fashion, in slot order.
 //
-// Per product, staging included, contexts' streams back to back, before -> after (dp2a kernel; mma.sync kernel with 16 rows per
-// CTA and every warp staging its own activations for Q6_K of two tokens and more):
-//   see the table at raw_mma_launch.
+// Time per product in microseconds, staging included, back to back in a CUDA graph (rate of the reference bytes at one token), and
+// in brackets the kernels before: dp2a on CUDA cores, and for Q6_K of two tokens and more an MMA kernel of 16 rows per CTA whose
+// warps staged the activations each for themselves:
+//   W[8192, 28672]   1 token            8 tokens     16 tokens         W[11008, 4096], 5 tokens
+//   Q6_K             50 (62)  3.9 TB/s   72 (100)    117 (135)         19
+//   Q5_K             44 (73)  3.6 TB/s   61          87 (590)          18 (61)
+//   Q8_K             53 (69)  5.0 TB/s   60          81                19
+//   Q4_0             38 (53)  3.4 TB/s   58          82 (590)          18
+//   Q5_0             51 (67)  3.2 TB/s   70          95 (590)          21
 #include "common.cuh"
 
 namespace gllmk {
@@ -429,8 +435,32 @@ __device__ __forceinline__ int rm_cta_of(const RmParams &p, int64_t u) {
     return u < big ? (int)(u / (p.per_cta + 1)) : p.rem + (int)((u - big) / p.per_cta);
 }
 
+// Adds the shares of TL tokens (t0, t0 + 2, ...) in slot order, SU slots' loads in flight at a time.
+template <int TL, int SU>
+__device__ __forceinline__ void rm_sum(const RmParams &p, const float *part, int t0, int nsl, float sc, float *y) {
+    float v[TL];
+#pragma unroll
+    for (int i = 0; i < TL; i++) v[i] = 0.0f;
+    for (int s = 0; s < nsl; s += SU) {
+        float q[SU][TL];
+#pragma unroll
+        for (int u = 0; u < SU; u++)
+#pragma unroll
+            for (int i = 0; i < TL; i++) q[u][i] = s + u < nsl && t0 + 2 * i < p.m ? __ldcg(part + (size_t)(s + u) * 256 + (t0 + 2 * i) * 16) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < SU; u++)
+#pragma unroll
+            for (int i = 0; i < TL; i++) v[i] += q[u][i];
+    }
+#pragma unroll
+    for (int i = 0; i < TL; i++)
+        if (t0 + 2 * i < p.m) y[(size_t)(t0 + 2 * i) * p.yst] = p.n_row_scales > 0 ? v[i] * sc : v[i];
+}
+
 // This warp's share of a row tile is complete: red[16][rp] holds its column sums.  The last contributing CTA adds the shares in
-// slot order and writes y.
+// slot order and writes y.  FEW (one or two tokens): a plain loop over the shares; the batches' registers, live across this call,
+// cost the one-group kernels 10 % of their whole time (Q4_0 W[8192, 28672] 38.7 against 42.4 us).
+template <bool FEW>
 __device__ __noinline__ void rm_flush(const RmParams &p, const float *red, int rp, int64_t tile, int slot, int nsl) {
     const int lane = threadIdx.x & 31, r = lane & 15, t0 = lane >> 4;
     float *base = p.partial + (size_t)tile * p.maxslot * 256;
@@ -454,16 +484,23 @@ __device__ __noinline__ void rm_flush(const RmParams &p, const float *red, int r
     float sc = 1.0f;
     if (p.n_row_scales == 1) sc = p.row_scales[0];
     else if (p.n_row_scales > 1) sc = p.row_scales[row];
+    float *y = p.y + (size_t)row * p.ysr;
+    if (nsl > 1) {
+        // one L2 round trip per batch, not per share (W[4096, 4096], 16 tokens, 15 shares per tile: 21 -> 18 us)
+        if (FEW) {
+            for (int tok = t0; tok < p.m; tok += 2) {
+                float v = 0.0f;
+                for (int s = 0; s < nsl; s++) v += __ldcg(base + (size_t)s * 256 + tok * 16 + r);
+                y[(size_t)tok * p.yst] = p.n_row_scales > 0 ? v * sc : v;
+            }
+        } else if (p.m <= 8) rm_sum<4, 4>(p, base + r, t0, nsl, sc, y);
+        else rm_sum<8, 4>(p, base + r, t0, nsl, sc, y);
+        return;
+    }
     for (int tok = t0; tok < p.m; tok += 2) {
-        float v = 0.0f;
-        if (nsl > 1) {
-            for (int s = 0; s < nsl; s++) v += __ldcg(base + (size_t)s * 256 + tok * 16 + r);
-        } else {
-            const float *c = red + r * rp + 3 * tok;
-            v = (c[2] + c[1]) + c[0];
-        }
-        if (p.n_row_scales > 0) v *= sc;
-        p.y[(size_t)tok * p.yst + (size_t)row * p.ysr] = v;
+        const float *c = red + r * rp + 3 * tok;
+        const float v = (c[2] + c[1]) + c[0];
+        y[(size_t)tok * p.yst] = p.n_row_scales > 0 ? v * sc : v;
     }
 }
 
@@ -480,7 +517,7 @@ __host__ __device__ constexpr int rm_min_ctas(int ng) { return ng <= 2 ? 3 : 2; 
 template <int QT, int NG>
 __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_kernel(const __grid_constant__ RmParams p) {
     using F = Rm<QT>;
-    constexpr int CH = F::CH, NCP = (16 * CH + 31) / 32;
+    constexpr int CH = F::CH;
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int ncol = 3 * p.m, S = p.stages, nb = p.nb;
@@ -492,30 +529,34 @@ __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_k
     const int n = p.per_cta + ((int)blockIdx.x < p.rem ? 1 : 0);
 
     // ---- copies: the producer's position runs S - 1 steps ahead of the consumer's ----
+    // Half a warp per row piece (a whole one for Q8_K's nineteen 16-byte chunks): lane = chunk, so a copy is one instruction and one
+    // addition (with chunk i = lane + 32 j of all sixteen pieces instead, the index arithmetic took a third of the kernel's
+    // instructions: Q6_K W[8192, 28672], one token 52 us)
     int64_t ptg = u0 / nb;
     int pb = (int)(u0 - ptg * nb);
-    const uint32_t wdst = base + 16 * warp * F::PITCH;
-    // this lane's copies: chunk i = lane + 32 j of the warp's 16 x CH: row i / CH (rows past the last one repeat it; not stored)
-    int rr[NCP];
-    const uint8_t *wtile = nullptr;  // nullptr: all of the warp's rows are past the last one
+    constexpr int LPR = CH > 16 ? 32 : 16, RPI = 32 / LPR;  // lanes per row piece, row pieces per instruction
+    const int hrow = lane / LPR, ch = lane % LPR;
+    const uint32_t wdst = base + (16 * warp + hrow) * F::PITCH + 16 * ch;
+    const uint8_t *wsrc = nullptr;  // this lane's chunk of the first row piece it copies
+    int rows = 0;                   // rows of the warp's tile inside the matrix
     const auto set_tile = [&]() {
         const int64_t row0 = ptg * RM_ROWS + 16 * warp;
-        wtile = row0 < p.n ? p.w + (size_t)row0 * p.pitch : nullptr;
-        const int last = row0 + 15 < p.n ? 15 : (int)(p.n - 1 - row0);
-#pragma unroll
-        for (int j = 0; j < NCP; j++) rr[j] = min((lane + 32 * j) / CH, last);
+        rows = row0 + 16 <= p.n ? 16 : (row0 < p.n ? (int)(p.n - row0) : 0);
+        wsrc = p.w + (size_t)(row0 + (hrow < rows ? hrow : 0)) * p.pitch + (size_t)pb * F::BYTES + 16 * ch;
     };
     const auto copy_rows = [&](int st) {
-        if (wtile) {
-            const uint8_t *src = wtile + (size_t)pb * F::BYTES;
-            const uint32_t dst = wdst + st * stage;
+        if (ch < CH) {
+            uint32_t dst = wdst + st * stage;
+            if (rows == 16) {
+                const uint8_t *src = wsrc;
 #pragma unroll
-            for (int j = 0; j < NCP; j++) {
-                const int i = lane + 32 * j;
-                if (16 * CH % 32 == 0 || j < NCP - 1 || i < 16 * CH) {
-                    uintptr_t a = reinterpret_cast<uintptr_t>(src) + (uint64_t)(uint32_t)rr[j] * p.pitch;
-                    if (!F::ALIGNED) a &= ~(uintptr_t)15;
-                    cp16(dst + (F::PITCH == 16 * CH ? 16 * i : (i / CH) * F::PITCH + (i % CH) * 16), reinterpret_cast<const uint8_t *>(a) + 16 * (i % CH));
+                for (int j = 0; j < 16 / RPI; j++, src += (size_t)RPI * p.pitch, dst += RPI * F::PITCH)
+                    cp16(dst, F::ALIGNED ? src : reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(src) & ~(uintptr_t)15));
+            } else {
+                // the matrix ends inside the tile: rows past the last one are not copied (what they yield is not stored)
+                for (int r = hrow; r < rows; r += RPI, dst += RPI * F::PITCH) {
+                    const uintptr_t src = reinterpret_cast<uintptr_t>(wsrc) + (size_t)(r - hrow) * p.pitch;
+                    cp16(dst, reinterpret_cast<const uint8_t *>(F::ALIGNED ? src : src & ~(uintptr_t)15));
                 }
             }
         }
@@ -526,6 +567,7 @@ __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_k
         for (uint32_t o = threadIdx.x * 16; o < slice; o += RM_WARPS * 32 * 16) cp16(dst + o, src + o);
     };
     const auto advance = [&]() {
+        wsrc += F::BYTES;
         if (++pb == nb) {
             pb = 0;
             ptg++;
@@ -577,11 +619,10 @@ __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_k
         if (row0 < p.n) {
             uint32_t r0 = base + st * stage + (16 * warp + g) * F::PITCH, r8 = r0 + 8 * F::PITCH;
             if (!F::ALIGNED) {
-                // where the block starts in its first 16 bytes (a surplus row reads the last row's bytes as that row has them)
-                const uint32_t w0 = (uint32_t)reinterpret_cast<uintptr_t>(p.w) + (uint32_t)b * F::BYTES;
-                const uint32_t ra = (uint32_t)(row0 + g < p.n ? row0 + g : p.n - 1), rb = (uint32_t)(row0 + g + 8 < p.n ? row0 + g + 8 : p.n - 1);
-                r0 += (w0 + ra * p.pitch) & 15u;
-                r8 += (w0 + rb * p.pitch) & 15u;
+                // where the block starts in its first 16 bytes
+                const uint32_t ra = (uint32_t)reinterpret_cast<uintptr_t>(p.w) + (uint32_t)b * F::BYTES + (uint32_t)(row0 + g) * p.pitch;
+                r0 += ra & 15u;
+                r8 += (ra + 8 * p.pitch) & 15u;
             }
             const uint32_t xs = base + st * stage + RM_ROWS * F::PITCH;
             RmCols x;
@@ -605,7 +646,7 @@ __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_k
                         tot[ng][j] = 0.0f;
                     }
                 __syncwarp();
-                rm_flush(p, red, 8 * NG + 1, tg * RM_WARPS + warp, (int)blockIdx.x - slot0, nsl);
+                rm_flush<NG == 1>(p, red, 8 * NG + 1, tg * RM_WARPS + warp, (int)blockIdx.x - slot0, nsl);
                 __syncwarp();
             }
             b = 0;
@@ -651,6 +692,11 @@ int32_t rm_pass(Ctx *c, RmParams &p, cudaStream_t s) {
     const int64_t groups = (p.n + RM_ROWS - 1) / RM_ROWS, units = groups * p.nb;
     int64_t ctas = (int64_t)c->sm_count * per_sm;
     if (ctas > units) ctas = units;
+    // few units per CTA: no more CTAs than the longest share needs — 512 units on 444 CTAs take as long as on 256 CTAs of two, whose
+    // tiles have half the shares to write, count and add up (W[4096, 4096]: 13.1 -> 12.2 us at 5 tokens, W[11008, 4096], four units:
+    // 15.7 -> 14.8).  With one or two tokens and two units the smaller grid is the slower one (10.2 against 10.6 us)
+    const int64_t longest = (units + ctas - 1) / ctas;
+    if (longest <= 4 && (longest > 2 || NG > 1)) ctas = (units + longest - 1) / longest;
     if (units / ctas > 0x3fffffff) return fail(c, GLLMK_STATUS_INVALID_ARG, "gemv: matrix too large");
     p.per_cta = (int)(units / ctas);
     p.rem = (int)(units % ctas);

@@ -429,3 +429,36 @@ def test_gemm_q8_against_the_oracle(gk, K, oracle, m, n, k, nscales):
     with pytest.raises(gk.GllmkError) as e:  # k % 256 != 0: the reference asserts
         K.gemm_q8(b.view(np.int8), x, out, None, m, n, 100)
     assert e.value.status == gk.Status.INVALID_ARG
+
+
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("n,k,m", [(1, 256, 1), (16, 512, 2), (127, 3 * 256, 3), (129, 7 * 256, 5), (130, 5 * 256, 6), (257, 19 * 256, 11), (1000, 33 * 256, 14)])
+def test_gemv_against_64_bit_product(K, gk, oracle, torch, name, n, k, m):
+    """The integer tensor-core GEMV at the edges of its tiles (128 rows per CTA, 16 per warp, columns in groups of eight = 2 2/3
+    tokens, shares of a row that several CTAs add up).  Activations are 24-bit fixed point per 256 elements (6e-8 of the block's
+    maximum), products exact, sums f32 over at most k / 256 blocks: 1e-6 of the result's norm is ten times what that gives."""
+    qt = qtype(gk, name)
+    blocks = random_blocks(name, qt, n, k, 900 + n + m)
+    x = np.random.default_rng(n + m).standard_normal((m, k)).astype(np.float32)
+    want = x.astype(np.float64) @ oracle_matrix(oracle, qt, blocks, n, k).reshape(n, k).astype(np.float64).T
+    w = K.upload(qt, n, k, blocks)
+    y = K.gemv(w, torch.from_numpy(x).cuda())
+    assert torch.equal(y, K.gemv(w, torch.from_numpy(x).cuda()))  # shares are added in a fixed order
+    y = y.cpu().numpy()
+    assert K.status() == 0
+    assert np.linalg.norm(y - want) <= 1e-6 * np.linalg.norm(want)
+    w.free()
+
+
+@pytest.mark.parametrize("name", ["q4_0", "q5_0"])
+@pytest.mark.parametrize("k", [256 + 32, 512 - 32])
+def test_gemv_rows_of_other_lengths_stay_on_the_dp2a_kernel(K, gk, oracle, torch, name, k):
+    qt = qtype(gk, name)
+    n, m = 37, 3
+    blocks = random_blocks(name, qt, n, k, 7)
+    x = np.random.default_rng(8).standard_normal((m, k)).astype(np.float32)
+    ref = oracle.quant_matmul(blocks, np.ascontiguousarray(x.T), qt.id, n, m, k, threads=2)
+    w = K.upload(qt, n, k, blocks)
+    y = K.gemv(w, torch.from_numpy(x).cuda()).cpu().numpy()
+    assert oracle.rel_err(y.T, ref) <= TOL
+    w.free()
