@@ -4,13 +4,15 @@
 //
 // Weight-only formats (Q4_K, Q8_0, MXFP4, NVFP4 weights with bf16/f32 activations), gemm_wq_kernel.
 // A CTA owns MT (1 or 2) tiles of 128 weight rows (UMMA M, one TMEM accumulator each) x up to 256 tokens
-// (UMMA N) and walks K in steps of 64 (64 fp16 = one 128-byte swizzle row).  With MT = 2 one activation tile
-// feeds two MMAs, which halves the shared-memory fill traffic per flop (the L2 -> SM path, not the tensor
-// core, is what bounds a 128 x 256 tile):
+// (UMMA N; 192 with MT = 2) and walks K in steps of 64 (64 fp16 = one 128-byte swizzle row).  With MT = 2 one
+// activation tile feeds two MMAs, which halves the shared-memory fill traffic per flop:
 //   * the RAW quantized weights of its 128 rows arrive as one bulk copy per 256 k ("super-chunk": the same
 //     contiguous byte range the decode GEMV streams) into a shared-memory ring, mbarrier-tracked;
 //   * four dequant warps turn a quarter of a super-chunk (64 k) into fp16 with packed half2 arithmetic and
-//     store it as the 128-byte-swizzled K-major operand A tile the tensor core reads;
+//     store it in tensor memory (tcgen05.st), from where the MMA takes operand A.  As a swizzled tile in shared
+//     memory it was written and read there once more, 256 of the ~480 cycles of shared-memory traffic that an A tile
+//     of a small batch cost (~750 at 256 tokens, against 540 of tensor-core time), and needed a proxy fence of ~150:
+//     W[28672, 8192] Q4_K x 33 tokens 80 us, now 59; x 512 tokens 201 us, now 195;
 //   * the activations were converted once per call to fp16 tile images (stage_act_kernel), so operand B
 //     of a k-step is one or two bulk copies of 16 KB;
 //   * one elected thread issues tcgen05.mma (kind::f16, f32 accumulate in TMEM); tcgen05.commit hands the
@@ -29,7 +31,11 @@ namespace gllmk {
 constexpr int WQ_BM = 128;         // weight rows per CTA (UMMA M)
 constexpr int WQ_BN = 256;         // tokens per CTA (UMMA N, <= 256)
 constexpr int WQ_TILE = 16384;     // one operand tile: 128 rows x 128 bytes
-constexpr int WQ_SA = 4;           // operand A (dequantized weight tiles) ring: one slot per dequant group
+constexpr int WQ_SA = 4;           // operand A (dequantized weight tiles) ring in tensor memory: one slot per dequant group
+constexpr uint32_t WQ_TMEM = 512;  // tensor-memory columns: accumulators, then the A ring (32 columns a tile)
+constexpr int WQ_BN2 = 192;        // tokens per CTA with two row tiles: 2 x 192 + 4 x 32 columns
+constexpr uint32_t WQ_ACC2 = WQ_BN2;
+__host__ __device__ constexpr uint32_t wq_a_col(int mt, int slot) { return (mt == 2 ? 2 * WQ_BN2 : 256) + 32u * (uint32_t)slot; }
 constexpr int WQ_MAX_SB = 12;      // operand B (activation) stages, at most
 constexpr int WQ_MAX_R = 8;        // raw super-chunk ring, at most
 constexpr int WQ_DW = 16;          // dequant warps
@@ -80,7 +86,7 @@ struct GemmParams {
     int y_bf16;
     int64_t ldy;
     int vec;             // Y allows 16-byte stores
-    int ntok;            // MMA N of this launch (multiple of 32, <= 256)
+    int ntok, ntok32;    // MMA N of this launch (multiple of 16; <= 192 with two row tiles, <= 256 with one); rounded up to 32
     int row_tiles;       // 128-row tiles of the weight matrix
     int sb, r;           // ring depths: B stages, raw super-chunks
     int *status;
@@ -99,7 +105,7 @@ struct GemmParams {
 __device__ __forceinline__ float swiglu_f32(float g, float u) { return (g / (1.0f + expf(-g))) * u; }
 __global__ void __launch_bounds__(256) stage_act_kernel(const void *__restrict__ a, int a_bf16, int64_t lda, int64_t k_valid,
                                                         uint8_t *__restrict__ xt, const __grid_constant__ ImgTiles imgs,
-                                                        const void *__restrict__ a_up) {
+                                                        const void *__restrict__ a_up, int quad_order) {
     // The GEMM behind this launch may start now (programmatic dependent launch): its CTAs take the SMs this grid leaves,
     // allocate tensor memory and stream raw weights; the one thread that reads these tile images orders itself after
     // this grid with griddepcontrol.wait.
@@ -151,7 +157,15 @@ __global__ void __launch_bounds__(256) stage_act_kernel(const void *__restrict__
                 o = make_uint4(r[0], r[1], r[2], r[3]);
             }
         }
-        *reinterpret_cast<uint4 *>(dst + tc::sw128_offset(row, chunk)) = o;
+        if (quad_order) {
+            // Q4_K / Q8_0 (store_quads): elements 8t .. 8t + 3 of a 32-element block are k' = 4t .. 4t + 3, elements 8t + 4 .. + 7
+            // k' = 16 + 4t .. + 3
+            const int c0 = (chunk & 4) + ((chunk & 3) >> 1), off = 8 * (chunk & 1);
+            *reinterpret_cast<uint2 *>(dst + tc::sw128_offset(row, c0) + off) = make_uint2(o.x, o.y);
+            *reinterpret_cast<uint2 *>(dst + tc::sw128_offset(row, c0 + 2) + off) = make_uint2(o.z, o.w);
+        } else {
+            *reinterpret_cast<uint4 *>(dst + tc::sw128_offset(row, chunk)) = o;
+        }
     }
 }
 
@@ -216,29 +230,25 @@ __device__ __forceinline__ __half2 scale_h2(float s) {
 // Q4_K / Q8_0: warp wg handles the 16-row chunks wg and wg + 4; its lane reads the uint4 the device layout
 // keeps for it (rows g and g + 8, bytes 8t..8t+7 of the 32-byte group) and produces, for both rows, the
 // 16-byte fp16 groups t (low nibbles / even block) and 4 + t (high nibbles / odd block).
-// Which of a chunk's row pairs (g, g + 8) a lane works on.  With g = lane / 4 the eight lanes that a 16-byte shared-memory
-// access handles together (lanes 8i .. 8i+7) would write rows g and g + 1 of the swizzled A tile, whose four 16-byte
-// groups (t ^ g) fall on the same four bank groups: a two-way conflict on every store.  Pairing rows q and q ^ 5 in such
-// an octet puts its eight stores on eight different bank groups and keeps its eight loads of the raw chunk (16-byte
-// slots 4g + t) on eight different ones as well.
-__device__ __forceinline__ int wq_row_of_lane(int lane) {
-    const int q = lane >> 3;
-    return (lane & 4) ? (q ^ 5) : q;
-}
-
-// Q4_K / Q8_0: the eight 16-byte groups a lane has made (o[4 * ci + 2 * h + {0, 1}] = groups t and 4 + t of row
-// 16 * (wg + 4 * ci) + 8 * h + g) go to the swizzled A tile
-__device__ __forceinline__ void store_kq(uint8_t *at, int wg, int lane, const uint4 (&o)[8]) {
-    const int g = wq_row_of_lane(lane), t = lane & 3;
+// Thread = weight row (FP4 and the row-major formats): the row's 64 elements are 32 columns of its tensor-memory lane.
+__device__ __forceinline__ void store_rows(uint32_t ta, const uint4 (&o)[8]) {
+    uint32_t r[32];
 #pragma unroll
-    for (int ci = 0; ci < 2; ci++)
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            uint8_t *rowp = at + (16 * (wg + 4 * ci) + 8 * h + g) * 128;  // (row & 7) == g
-            *reinterpret_cast<uint4 *>(rowp + ((t ^ g) << 4)) = o[4 * ci + 2 * h];
-            *reinterpret_cast<uint4 *>(rowp + (((4 + t) ^ g) << 4)) = o[4 * ci + 2 * h + 1];
-        }
+    for (int c = 0; c < 8; c++) r[4 * c] = o[c].x, r[4 * c + 1] = o[c].y, r[4 * c + 2] = o[c].z, r[4 * c + 3] = o[c].w;
+    tc::tmem_st32(ta, r);
 }
+// Q4_K / Q8_0: o[4 ci + 2 h + {0, 1}] are elements 8t .. 8t + 7 of the step's first and second 32-element block, row 16 ci + 8 h + g of
+// the warp's 32.  The 16-lane store takes, per group of eight columns, columns 2t and 2t + 1 from thread t, so a block's element
+// pairs 0, 1 go to its first eight columns and 2, 3 to its second eight: an order of k that the activation images repeat.
+__device__ __forceinline__ void store_quads(uint32_t ta, const uint4 (&o)[8]) {
+#pragma unroll
+    for (int ci = 0; ci < 2; ci++) {
+        const uint4 &l0 = o[4 * ci], &h0 = o[4 * ci + 1], &l8 = o[4 * ci + 2], &h8 = o[4 * ci + 3];
+        const uint32_t r[16] = {l0.x, l0.y, l8.x, l8.y, l0.z, l0.w, l8.z, l8.w, h0.x, h0.y, h8.x, h8.y, h0.z, h0.w, h8.z, h8.w};
+        tc::tmem_st16x256_x4(ta + ((uint32_t)(16 * ci) << 16), r);
+    }
+}
+constexpr bool wq_quads(int fmt) { return fmt == FMT_Q4K || fmt == FMT_Q80; }
 
 template <int FMT>
 struct Dequant;
@@ -247,12 +257,12 @@ template <>
 struct Dequant<FMT_Q4K> {
     float global;
     __device__ __forceinline__ void compute(const uint8_t *raw, int p, int wg, int lane, uint4 (&o)[8]) {
-        const int g = wq_row_of_lane(lane), t = lane & 3, vl = 4 * g + t;
+        const int g = lane >> 2, t = lane & 3;
         // (d*sc, -dmin*m) of sub-blocks 2p and 2p+1: lane t works them out for (chunk, row) pair t of the four
         // pairs its quad shares; everyone fetches all four pairs with shuffles
         __half2 mine_lo, mine_hi;
         {
-            const uint8_t *chunk = raw + (wg + 4 * (t >> 1)) * Q4K_CHUNK;
+            const uint8_t *chunk = raw + (2 * wg + (t >> 1)) * Q4K_CHUNK;
             const int h = t & 1, rr = g + 8 * h;
             const uint32_t dd = *reinterpret_cast<const uint32_t *>(chunk + 2304 + (g * 2 + h) * 4);
             const float d = __half2float(__ushort_as_half((unsigned short)(dd & 0xFFFFu)));
@@ -264,8 +274,8 @@ struct Dequant<FMT_Q4K> {
         }
 #pragma unroll
         for (int ci = 0; ci < 2; ci++) {
-            const int c = wg + 4 * ci;
-            const uint4 q = *reinterpret_cast<const uint4 *>(raw + c * Q4K_CHUNK + (p * 32 + vl) * 16);
+            const int c = 2 * wg + ci;
+            const uint4 q = *reinterpret_cast<const uint4 *>(raw + c * Q4K_CHUNK + (p * 32 + lane) * 16);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int src = (lane & ~3) | (2 * ci + h);
@@ -277,20 +287,19 @@ struct Dequant<FMT_Q4K> {
             }
         }
     }
-    __device__ __forceinline__ void store(uint8_t *at, int wg, int lane, const uint4 (&o)[8]) { store_kq(at, wg, lane, o); }
 };
 
 template <>
 struct Dequant<FMT_Q80> {
     float global;
     __device__ __forceinline__ void compute(const uint8_t *raw, int p, int wg, int lane, uint4 (&o)[8]) {
-        const int g = wq_row_of_lane(lane), t = lane & 3, vl = 4 * g + t;
+        const int g = lane >> 2, t = lane & 3;
 #pragma unroll
         for (int ci = 0; ci < 2; ci++) {
-            const int c = wg + 4 * ci;
+            const int c = 2 * wg + ci;
             const uint8_t *chunk = raw + c * Q80_CHUNK;
-            const uint4 q0 = *reinterpret_cast<const uint4 *>(chunk + ((2 * p) * 32 + vl) * 16);
-            const uint4 q1 = *reinterpret_cast<const uint4 *>(chunk + ((2 * p + 1) * 32 + vl) * 16);
+            const uint4 q0 = *reinterpret_cast<const uint4 *>(chunk + ((2 * p) * 32 + lane) * 16);
+            const uint4 q1 = *reinterpret_cast<const uint4 *>(chunk + ((2 * p + 1) * 32 + lane) * 16);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int rr = g + 8 * h;
@@ -303,7 +312,6 @@ struct Dequant<FMT_Q80> {
             }
         }
     }
-    __device__ __forceinline__ void store(uint8_t *at, int wg, int lane, const uint4 (&o)[8]) { store_kq(at, wg, lane, o); }
 };
 
 // FP4: the raw super-chunk is the row tile's swizzled data image (16 KB) followed by its scale atoms (512 B
@@ -328,12 +336,6 @@ struct DequantFp4 {
         }
 #pragma unroll
         for (int c = 0; c < 8; c++) o[c] = fp4_word(w[c], s[c >> 1]);
-    }
-    __device__ __forceinline__ void store(uint8_t *at, int wg, int lane, const uint4 (&o)[8]) {
-        const int r = 32 * wg + lane;
-        uint8_t *rowp = at + r * 128;
-#pragma unroll
-        for (int c = 0; c < 8; c++) *reinterpret_cast<uint4 *>(rowp + ((c ^ (r & 7)) << 4)) = o[c];
     }
 };
 template <>
@@ -392,12 +394,6 @@ struct Dequant<FMT_Q6K> {
             }
         }
     }
-    __device__ __forceinline__ void store(uint8_t *at, int wg, int lane, const uint4 (&o)[8]) {
-        const int r = 32 * wg + lane;
-        uint8_t *rowp = at + r * 128;
-#pragma unroll
-        for (int c = 0; c < 8; c++) *reinterpret_cast<uint4 *>(rowp + ((c ^ (r & 7)) << 4)) = o[c];
-    }
 };
 
 // Q5_K (k_quant.rs:381-436): d f16 @0, dmin f16 @2, scales[12] @4, qh[32] @16, qs[128] @48.  Thread = weight row.  k-step p
@@ -441,12 +437,6 @@ struct Dequant<FMT_Q5K> {
                     out = make_uint4(r[0], r[1], r[2], r[3]);
                 }
         }
-    }
-    __device__ __forceinline__ void store(uint8_t *at, int wg, int lane, const uint4 (&o)[8]) {
-        const int r = 32 * wg + lane;
-        uint8_t *rowp = at + r * 128;
-#pragma unroll
-        for (int c = 0; c < 8; c++) *reinterpret_cast<uint4 *>(rowp + ((c ^ (r & 7)) << 4)) = o[c];
     }
 };
 
@@ -500,12 +490,6 @@ struct DequantClassic {
                 }
         }
     }
-    __device__ __forceinline__ void store(uint8_t *at, int wg, int lane, const uint4 (&o)[8]) {
-        const int r = 32 * wg + lane;
-        uint8_t *rowp = at + r * 128;
-#pragma unroll
-        for (int c = 0; c < 8; c++) *reinterpret_cast<uint4 *>(rowp + ((c ^ (r & 7)) << 4)) = o[c];
-    }
 };
 template <>
 struct Dequant<FMT_Q40> : DequantClassic<FMT_Q40> {};
@@ -539,11 +523,10 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
     __shared__ uint32_t tmem_base_s;
     __shared__ int abort_s;
     constexpr int RAW = wq_raw_bytes(FMT);
-    constexpr uint32_t TMEM_COLS = MT == 2 ? 512 : 256;
     const uint32_t smem_s = (tc::smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem = smem_raw + (smem_s - tc::smem_u32(smem_raw));
     const int bstage = p.ntok * 128;
-    const uint32_t a_off = 0, b_off = (uint32_t)(WQ_SA * WQ_TILE), raw_off = b_off + (uint32_t)(p.sb * bstage);
+    const uint32_t b_off = 0, raw_off = (uint32_t)(p.sb * bstage);
     const uint32_t fullA = tc::smem_u32(&bars[0]), emptyA = fullA + 8 * WQ_SA, fullB = emptyA + 8 * WQ_SA,
                    emptyB = fullB + 8 * WQ_MAX_SB, rawfull = emptyB + 8 * WQ_MAX_SB, rawempty = rawfull + 8 * WQ_MAX_R,
                    accum = rawempty + 8 * WQ_MAX_R;
@@ -588,7 +571,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
         tc::mbar_init(accum, (uint32_t)mt);
         tc::mbar_init_fence();
     }
-    if (warp == 2) tc::tmem_alloc(tc::smem_u32(&tmem_base_s), TMEM_COLS);
+    if (warp == 2) tc::tmem_alloc(tc::smem_u32(&tmem_base_s), WQ_TMEM);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -691,38 +674,43 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
             }
         }
     } else if (warp < WQ_CTRL) {
-        // ---------------- MMA issue: one thread per row tile ----------------
-        // Every step of this role (barrier probe, fence, MMA, commit) has a long issue latency, ~0.9 k cycles per A tile
-        // in all, against 0.25 - 0.5 k cycles of tensor-pipe time: with two row tiles, two threads in two warps — each with
-        // its own accumulator and its own A slots (tile a = 2 * ks + i lives in slot a % 4) — keep the pipe fed.
-        const int i = warp - 2;
-        if (lane == 0 && i < mt) {
+        // ---------------- MMA issue: one warp per row tile ----------------
+        // With two row tiles, two warps — each with its own accumulator and its own A slots (tile a = 2 * ks + i lives in slot a % 4).
+        // The whole warp walks the steps and one elected lane issues: addresses and descriptors are then uniform values; with a
+        // single active lane the four MMAs of a step took ~320 cycles to issue and the step 780, which paced every tile below
+        // 128 tokens.
+        const int i = __shfl_sync(0xffffffffu, warp, 0) - 2;
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_d, 0);
+        if (i < mt) {
             const uint32_t idesc = tc::idesc_f16(WQ_BM, p.ntok, 0, 0);  // fp16 x fp16 -> f32
             bool ok = true;
             int sb = 0, bround = 0;
-            for (int ks = 0; ks < nks && ok; ks++) {
+            for (int ks = 0; ks < nks; ks++) {
                 WQP_T0();
                 const uint64_t bd = tc::smem_desc_sw128(smem_s + b_off + (uint32_t)(sb * bstage));
                 const int a = ks * mt + i, sa = a % WQ_SA;
                 // probes that do not suspend the thread: its reaction time is on the critical path of every tile
-                ok = tc::mbar_spin(fullB + 8 * sb, (uint32_t)(bround & 1), abort_flag) &&
-                     tc::mbar_spin(fullA + 8 * sa, (uint32_t)((a / WQ_SA) & 1), abort_flag);
+                ok = tc::mbar_spin_warp(fullB + 8 * sb, (uint32_t)(bround & 1), abort_flag) &&
+                     tc::mbar_spin_warp(fullA + 8 * sa, (uint32_t)((a / WQ_SA) & 1), abort_flag);
                 WQP_ACC(0);
                 if (!ok) {
                     abort_s = 1;
-                    atomicExch(p.status, 12);
+                    if (lane == 0) atomicExch(p.status, 12);
                     break;
                 }
                 tc::fence_after_sync();
-                const uint64_t ad = tc::smem_desc_sw128(smem_s + a_off + sa * WQ_TILE);
+                if (tc::elect_one()) {
 #pragma unroll
-                for (int k4 = 0; k4 < 4; k4++)
-                    tc::mma_f16(tmem_d + 256u * (uint32_t)i, ad + 2 * k4, bd + 2 * k4, idesc, (uint32_t)((ks | k4) != 0));
-                tc::mma_commit(emptyA + 8 * sa);  // the A tile is free when these MMAs have read it
-                tc::mma_commit(emptyB + 8 * sb);  // the stage, when both issuers' MMAs have
+                    for (int k4 = 0; k4 < 4; k4++)
+                        tc::mma_f16_ta(tmem_u + WQ_ACC2 * (uint32_t)i, tmem_u + wq_a_col(MT, sa) + 8u * k4, bd + 2 * k4, idesc, (uint32_t)((ks | k4) != 0));
+                    tc::mma_commit(emptyA + 8 * sa);  // the A tile is free when these MMAs have read it
+                    tc::mma_commit(emptyB + 8 * sb);  // the stage, when both issuers' MMAs have
+                    if (ks == nks - 1) tc::mma_commit(accum);
+                }
+                __syncwarp();
+                WQP_ACC(1);
                 if (++sb == p.sb) sb = 0, bround++;
             }
-            if (ok) tc::mma_commit(accum);
         }
     } else {
         // ---------------- dequant warps, then epilogue ----------------
@@ -773,9 +761,13 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
             WQP_ACC(3);
             ok = !*abort_flag;
             if (!ok) break;
-            dq.store(smem + a_off + grp * WQ_TILE, wg, lane, o);
+            tc::fence_after_sync();  // behind the MMAs that read the slot before
+            const uint32_t ta = tmem_d + ((uint32_t)(32 * wg) << 16) + wq_a_col(MT, grp);
+            if (wq_quads(FMT)) store_quads(ta, o);
+            else store_rows(ta, o);
             WQP_ACC(4);
-            tc::fence_proxy_async();  // every writer makes its own stores visible to the tensor core's proxy
+            tc::tmem_st_wait();
+            tc::fence_before_sync();
             WQP_ACC(5);
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(fullA + 8 * grp);
@@ -792,14 +784,14 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
             // every fourth group of 32 token columns
             tc::fence_after_sync();
             const int quad = warp & 3;
-            // all MMAs have completed, so the rings are free: each warp stages its blocks in 4 KB of the A ring
-            uint8_t *stage = smem + a_off + dw * 4096;
+            // all MMAs have completed, so the rings are free: each warp stages its blocks in 4 KB of them
+            uint8_t *stage = smem + dw * 4096;
             if (nsplit == 1) {
                 for (int i = 0; i < mt; i++) {
                     const int64_t row_base = (int64_t)(tile0 + i) * WQ_BM + 32 * quad;
-                    for (int c = 32 * (dw >> 2); c < p.ntok; c += 32 * (WQ_DW / 4)) {
+                    for (int c = 32 * (dw >> 2); c < p.ntok32; c += 32 * (WQ_DW / 4)) {
                         uint32_t v[32];
-                        tc::tmem_ld32(tmem_d + ((uint32_t)(32 * quad) << 16) + 256u * (uint32_t)i + (uint32_t)c, v);
+                        tc::tmem_ld32(tmem_d + ((uint32_t)(32 * quad) << 16) + WQ_ACC2 * (uint32_t)i + (uint32_t)c, v);
                         tc::tmem_ld_wait();
                         float o[32];
 #pragma unroll
@@ -812,14 +804,14 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
                 // A unit of a split tile: the accumulator goes to this unit's partial area ([row tile][token][128 rows]
                 // f32), and the unit that arrives last at the tile's counter adds the partials in unit order — the
                 // result does not depend on which one that is — and stores y.
-                const size_t unit_floats = (size_t)MT * p.ntok * WQ_BM;
+                const size_t unit_floats = (size_t)MT * p.ntok32 * WQ_BM;
                 float *tile_part = p.partial + (size_t)tail_tile * nsplit * unit_floats, *mine = tile_part + (size_t)split * unit_floats;
                 for (int i = 0; i < mt; i++)
-                    for (int c = 32 * (dw >> 2); c < p.ntok; c += 32 * (WQ_DW / 4)) {
+                    for (int c = 32 * (dw >> 2); c < p.ntok32; c += 32 * (WQ_DW / 4)) {
                         uint32_t v[32];
-                        tc::tmem_ld32(tmem_d + ((uint32_t)(32 * quad) << 16) + 256u * (uint32_t)i + (uint32_t)c, v);
+                        tc::tmem_ld32(tmem_d + ((uint32_t)(32 * quad) << 16) + WQ_ACC2 * (uint32_t)i + (uint32_t)c, v);
                         tc::tmem_ld_wait();
-                        float *dst = mine + ((size_t)i * p.ntok + c) * WQ_BM + 32 * quad + lane;
+                        float *dst = mine + ((size_t)i * p.ntok32 + c) * WQ_BM + 32 * quad + lane;
 #pragma unroll
                         for (int jj = 0; jj < 32; jj++) __stcg(dst + (size_t)jj * WQ_BM, __uint_as_float(v[jj]));  // lanes: 32 consecutive rows
                     }
@@ -836,12 +828,12 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
                 if (last_s) {
                     for (int i = 0; i < mt; i++) {
                         const int64_t row_base = (int64_t)(tile0 + i) * WQ_BM + 32 * quad;
-                        for (int c = 32 * (dw >> 2); c < p.ntok; c += 32 * (WQ_DW / 4)) {
+                        for (int c = 32 * (dw >> 2); c < p.ntok32; c += 32 * (WQ_DW / 4)) {
                             float o[32];
 #pragma unroll
                             for (int jj = 0; jj < 32; jj++) o[jj] = 0.0f;
                             for (int sp = 0; sp < nsplit; sp++) {
-                                const float *src = tile_part + (size_t)sp * unit_floats + ((size_t)i * p.ntok + c) * WQ_BM + 32 * quad + lane;
+                                const float *src = tile_part + (size_t)sp * unit_floats + ((size_t)i * p.ntok32 + c) * WQ_BM + 32 * quad + lane;
 #pragma unroll
                                 for (int jj = 0; jj < 32; jj++) o[jj] += __ldcg(src + (size_t)jj * WQ_BM);
                             }
@@ -859,7 +851,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
     WQP_OUT();
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 2) tc::tmem_dealloc(tmem_d, TMEM_COLS);
+    if (warp == 2) tc::tmem_dealloc(tmem_d, WQ_TMEM);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -890,12 +882,61 @@ static int32_t launch_wq_mt(Ctx *c, const GemmParams &p, const GemmGroups &G, in
     return mt == 2 ? launch_wq<FMT, 2>(c, p, G, grid, smem, s) : launch_wq<FMT, 1>(c, p, G, grid, smem, s);
 }
 
+// ---- which tile, how many of them side by side, and how the last wave is cut: estimated times, in microseconds ----
+// A k-step (64 k) of one unit, measured on W[37888, 4096 .. 8192] (one and two whole waves of 148 units; differences between the two
+// k, so without prologue and epilogue):
+//   tokens                     32    64   128   160   192   256
+//   one row tile,  Q4_K       .33   .33   .36   .45   .47   .51      (Q8_0 .49 - .56 from 128 tokens on, Q6_K .37 - .56)
+//   two row tiles, Q4_K       .40   .42   .49   .59   .65    -       (MXFP4 .36 - .60, Q8_0 .39 - .74, Q6_K .63 - .80)
+// Up to 128 tokens the dequant warps set the pace, from there on the tensor core (192 tokens x 2: 1.4 PFLOP/s).
+static double wq_step_us(int fmt, int mt, int ntok) {
+    if (mt == 1) {
+        const double t = ntok <= 128 ? 0.32 + 0.0003 * ntok : 0.40 + 0.00045 * ntok;
+        return t + (fmt == FMT_Q80 || wq_row_major(fmt) ? 0.03 : 0.0);
+    }
+    const double t = ntok <= 128 ? 0.375 + 0.0009 * ntok : 0.23 + 0.0022 * ntok;
+    if (wq_row_major(fmt)) return t + 0.16;
+    if (fmt == FMT_Q80) return t + 0.0005 * ntok;
+    return fmt == FMT_Q4K ? t : t - 0.05;
+}
+constexpr double WQ_UNIT_US = 4.0, WQ_CUT_US = 6.5;  // prologue and epilogue of a whole tile; of a tile's part
+// Time of `ntiles` token tiles of `ntok` tokens with `mt` row tiles per CTA.  The last — or only — wave, when it fills a fraction of
+// the SMs, is cut along k into *split units per tile, each with at least four k-blocks; the units' f32 partial sums are written by
+// each and read back by one of them (45 GB/s per SM fits what cut tiles measure: W[28672, 8192] Q6_K x 33 tokens, 112 pairs of row
+// tiles, 83 us whole and 106 us in fifths; W[11008, 4096] Q4_K x 256 tokens, 86 tiles, 37 us whole and 50 us in thirds).
+static double wq_estimate(const Ctx *c, int fmt, int nsc, int row_tiles, int ntiles, int ntok, int mt, int *split) {
+    const double tile_us = 4.0 * nsc * wq_step_us(fmt, mt, ntok), part_us = (double)mt * ntok * WQ_BM * 4.0 / 45e3;
+    const int sms = c->sm_count, units = ntiles * ((row_tiles + mt - 1) / mt), full = units / sms, tail = units - full * sms;
+    *split = 1;
+    double tail_us = tail > 0 ? tile_us + WQ_UNIT_US : 0.0;
+    if (tail > 0 && c->gemm_tail_split != 1)
+        for (int sp = 2; sp <= 8 && nsc / sp >= 4; sp++) {
+            const double t = (double)((tail * sp + sms - 1) / sms) * (tile_us / sp + WQ_CUT_US) + (sp + 1) * part_us;
+            if (t < tail_us) tail_us = t, *split = sp;
+        }
+    return full * (tile_us + WQ_UNIT_US) + tail_us;
+}
+// two row tiles share an activation stage and need two accumulators beside the A ring in tensor memory
+static bool wq_pairs(int row_tiles, int ntok) { return row_tiles % 2 == 0 && ntok <= WQ_BN2; }
+static int wq_format(const Weight *w) {
+    switch (w->qt) {
+        case GLLMK_QUANT_Q4K: return FMT_Q4K;
+        case GLLMK_QUANT_Q8_0: return FMT_Q80;
+        case GLLMK_QUANT_NVFP4: return FMT_NVFP4;
+        case GLLMK_QUANT_Q6_K: return FMT_Q6K;
+        case GLLMK_QUANT_Q5_K: return FMT_Q5K;
+        case GLLMK_QUANT_Q4_0: return FMT_Q40;
+        case GLLMK_QUANT_Q5_0: return FMT_Q50;
+        default: return FMT_MXFP4;
+    }
+}
+
 // One launch: groups [g0, g1) with their token ranges cut into tiles of `ntok` tokens.
 static int32_t gemm_groups_chunk(Ctx *c, const Weight *const *ws, int ng, const void *a, int a_bf16, int64_t lda,
                                  const int64_t *tok_begin, const int64_t *tok_count, int ntok, void *y, int y_bf16, int64_t ldy,
                                  cudaStream_t s, const void *a_up) {
     const Weight *w = ws[0];
-    const int fmt = w->qt == GLLMK_QUANT_Q4K ? FMT_Q4K : (w->qt == GLLMK_QUANT_Q8_0 ? FMT_Q80 : (w->qt == GLLMK_QUANT_NVFP4 ? FMT_NVFP4 : (w->qt == GLLMK_QUANT_Q6_K ? FMT_Q6K : (w->qt == GLLMK_QUANT_Q5_K ? FMT_Q5K : (w->qt == GLLMK_QUANT_Q4_0 ? FMT_Q40 : (w->qt == GLLMK_QUANT_Q5_0 ? FMT_Q50 : FMT_MXFP4))))));
+    const int fmt = wq_format(w);
     const int raw = wq_raw_bytes(fmt);
     GemmParams p{};
     GemmGroups G{};
@@ -908,6 +949,7 @@ static int32_t gemm_groups_chunk(Ctx *c, const Weight *const *ws, int ng, const 
     p.vec = (((uintptr_t)y & 15) == 0 && (ldy * (y_bf16 ? 2 : 4)) % 16 == 0) ? 1 : 0;
     p.status = c->status_dev;
     p.ntok = ntok;
+    p.ntok32 = (ntok + 31) / 32 * 32;
     const int halves = (ntok + 127) / 128;
     int ntiles = 0, nimg = 0;
     for (int g = 0; g < ng; g++) {
@@ -931,54 +973,37 @@ static int32_t gemm_groups_chunk(Ctx *c, const Weight *const *ws, int ng, const 
     if (ntiles == 0) return GLLMK_STATUS_OK;
     const int row_tiles = (int)((w->n_pad + WQ_BM - 1) / WQ_BM);  // (Q6_K rows are not padded on the device)
     const int bstage = ntok * 128;
-    // Row tiles per CTA and how the last wave is cut along k, chosen together.  Two row tiles share one activation stage
-    // (less shared-memory fill traffic per flop, two issuing threads, fixed costs paid once) but halve the CTA count; a
-    // last — or only — wave that fills a fraction of the SMs is cut along k into units (tail split, below).  Estimated
-    // time, in k-steps of a single tile: whole waves + the tail, times (k-steps per CTA x relative step cost + a fixed
-    // prologue / epilogue worth ~16 steps).
     const int sms = c->sm_count;
-    const auto estimate = [&](int m_t, int *split) -> double {
-        const double step = m_t == 2 ? 2.0 * (ntok > 128 ? 0.68 : 0.62) : 1.0;  // measured: a pair step costs 1.36 / 1.24 single steps
-        const int tiles = ntiles * ((row_tiles + m_t - 1) / m_t), full = tiles / sms, tail = tiles - full * sms;
-        double tail_t = tail > 0 ? 1.0 : 0.0;
-        *split = 1;
-        if (tail > 0 && c->gemm_tail_split != 1)
-            for (int sp = 2; sp <= 8 && p.nsc / sp >= 4; sp++) {
-                const double t = (double)((tail * sp + sms - 1) / sms) / sp + 0.05 * sp;  // + fill / drain and the partial traffic
-                if (t < tail_t) tail_t = t, *split = sp;
-            }
-        return (full + tail_t) * (4.0 * p.nsc * step + 16.0);
-    };
     int mt = 1;
-    if (row_tiles % 2 == 0) {
+    if (wq_pairs(row_tiles, ntok)) {
         int s1, s2;
-        if (estimate(2, &s2) < estimate(1, &s1)) mt = 2;
+        if (wq_estimate(c, fmt, p.nsc, row_tiles, ntiles, ntok, 2, &s2) < wq_estimate(c, fmt, p.nsc, row_tiles, ntiles, ntok, 1, &s1)) mt = 2;
         if (c->gemm_row_tiles == 1 || c->gemm_row_tiles == 2) mt = (int)c->gemm_row_tiles;
     }
-    // Shared-memory plan: four A tiles; three B stages (activation tiles come from L2: ~1 us of latency against
+    // Shared-memory plan (the A tiles are in tensor memory): three B stages (activation tiles come from L2: ~1 us of latency against
     // 0.2 - 0.5 us per k-step); everything else goes to the raw ring, because the weight stream comes from HBM and
     // with few tokens a k-step is short: two super-chunks in flight per SM cap the stream at ~15 GB/s per SM.
     p.sb = 3;
-    p.r = (WQ_SMEM_LIMIT - WQ_SA * WQ_TILE - p.sb * bstage) / raw;
+    p.r = (WQ_SMEM_LIMIT - p.sb * bstage) / raw;
     if (p.r < mt + 1) {  // big raw super-chunks (Q8_0) with a 256-token tile
         p.sb = 2;
-        p.r = (WQ_SMEM_LIMIT - WQ_SA * WQ_TILE - p.sb * bstage) / raw;
+        p.r = (WQ_SMEM_LIMIT - p.sb * bstage) / raw;
         if (p.r < mt + 1) mt = 1;
     }
     if (p.r > WQ_MAX_R) p.r = WQ_MAX_R;
     if (c->gemm_raw_slots >= mt + 1 && c->gemm_raw_slots < p.r) p.r = (int)c->gemm_raw_slots;
     if (p.r < mt + 1) return fail(c, GLLMK_STATUS_RUNTIME_ERROR, "gemm: shared-memory plan does not fit");
     // what the raw ring cannot use goes back to B stages
-    const int more_sb = (WQ_SMEM_LIMIT - WQ_SA * WQ_TILE - p.r * raw) / bstage;
+    const int more_sb = (WQ_SMEM_LIMIT - p.r * raw) / bstage;
     p.sb = more_sb > WQ_MAX_SB ? WQ_MAX_SB : more_sb;
-    const size_t smem = 1024 + (size_t)WQ_SA * WQ_TILE + (size_t)p.sb * bstage + (size_t)p.r * raw;
+    const size_t smem = 1024 + (size_t)p.sb * bstage + (size_t)p.r * raw;
     p.row_tiles = row_tiles;
     // activations -> fp16 tile images in the context's scratch
     const int nks = 4 * p.nsc;
     int32_t rc = ensure_act(c, (size_t)nimg * nks * WQ_TILE);
     if (rc) return rc;
     p.xt = static_cast<const uint8_t *>(c->act);
-    stage_act_kernel<<<dim3((unsigned)nks, (unsigned)nimg), 256, 0, s>>>(a, a_bf16, lda, w->k, static_cast<uint8_t *>(c->act), imgs, a_up);
+    stage_act_kernel<<<dim3((unsigned)nks, (unsigned)nimg), 256, 0, s>>>(a, a_bf16, lda, w->k, static_cast<uint8_t *>(c->act), imgs, a_up, wq_quads(fmt) ? 1 : 0);
     GK_CUDA(c, cudaGetLastError());
     dim3 grid((unsigned)ntiles, (unsigned)((row_tiles + mt - 1) / mt));
     // Tail split: the last, partly filled wave of tiles — the only one, when there are fewer tiles than SMs — is cut along
@@ -990,10 +1015,10 @@ static int32_t gemm_groups_chunk(Ctx *c, const Weight *const *ws, int ng, const 
         const int tiles = (int)(grid.x * grid.y);
         const int full = tiles / sms * sms, tail = tiles - full;
         int best_s = 1;
-        estimate(mt, &best_s);
+        (void)wq_estimate(c, fmt, p.nsc, row_tiles, ntiles, ntok, mt, &best_s);
         if (c->gemm_tail_split > 1 && p.nsc / (int)c->gemm_tail_split >= 1) best_s = (int)c->gemm_tail_split;
         if (tail > 0 && best_s > 1) {
-            const size_t unit_floats = (size_t)mt * ntok * WQ_BM;
+            const size_t unit_floats = (size_t)mt * p.ntok32 * WQ_BM;
             rc = ensure_red(c, (size_t)tail * best_s * unit_floats * sizeof(float));
             if (!rc) rc = ensure_cnt(c, (size_t)(tail + 1) * sizeof(int));
             if (rc) return rc;
@@ -1027,11 +1052,30 @@ int32_t gemm_grouped_launch(Ctx *c, const Weight *const *ws, int n_groups, const
         return fail(c, GLLMK_STATUS_UNSUPPORTED, "gemm: weight type %d is not block-quantized (use gllmk_gemm_int8)", ws[0]->qt);
     if (((uintptr_t)a & 15) || (lda % align)) return fail(c, GLLMK_STATUS_INVALID_ARG, "gemm: activations must be 16-byte aligned rows");
     if (ws[0]->k % 8) return fail(c, GLLMK_STATUS_INVALID_ARG, "gemm: k=%lld is not a multiple of 8", (long long)ws[0]->k);
-    // MMA N: 256-token tiles, or the largest group rounded up to a multiple of 32 when no group has more
+    // MMA N: the largest group in as many equal tiles of at most 256 tokens (a multiple of 16) as the estimate likes best
     int64_t most = 0;
     for (int g = 0; g < n_groups; g++) most = most > row_offsets[g + 1] - row_offsets[g] ? most : row_offsets[g + 1] - row_offsets[g];
     if (most <= 0) return GLLMK_STATUS_OK;
-    const int ntok = most >= WQ_BN ? WQ_BN : (int)((most + 31) / 32 * 32);
+    int ntok = 0;
+    {
+        const int fmt = wq_format(ws[0]), nsc = (int)((ws[0]->k + 255) / 256), row_tiles = (int)((ws[0]->n_pad + WQ_BM - 1) / WQ_BM);
+        const int64_t fewest = (most + WQ_BN - 1) / WQ_BN;
+        double best = 0.0;
+        for (int64_t t = fewest; t <= 2 * fewest + 1 && (t == fewest || most > 64 * t); t++) {
+            const int cand = (int)(((most + t - 1) / t + 15) / 16 * 16);
+            int64_t tiles = 0;
+            for (int g = 0; g < n_groups; g++) tiles += (row_offsets[g + 1] - row_offsets[g] + cand - 1) / cand;
+            if (tiles > 1 << 20) tiles = 1 << 20;
+            for (int m_t = 1; m_t <= (wq_pairs(row_tiles, cand) ? 2 : 1); m_t++) {
+                if (m_t == 1 && c->gemm_row_tiles == 2 && wq_pairs(row_tiles, cand)) continue;
+                if (m_t == 2 && c->gemm_row_tiles == 1) continue;
+                int sp;
+                const double us = wq_estimate(c, fmt, nsc, row_tiles, (int)tiles, cand, m_t, &sp);
+                if (ntok == 0 || us < best) best = us, ntok = cand;
+            }
+            if (t - fewest >= 8) break;  // many tiles: they no longer differ by much
+        }
+    }
     const int halves = (ntok + 127) / 128;
     // launches of at most WQ_MAX_GROUPS groups, WQ_MAX_TOK_TILES token tiles, WQ_MAX_IMG_TILES images
     const Weight *cw[WQ_MAX_GROUPS];
