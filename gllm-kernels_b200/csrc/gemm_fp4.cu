@@ -327,53 +327,63 @@ gemm_fp4_pair_kernel(const __grid_constant__ Fp4Params p, const int row_tiles, c
                 }
                 tc::mbar_arrive_cluster_relaxed(tc::map_to_cta(full2 + 8 * s, 0));
             }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && rank == 0) {
         // ---------------- leader CTA: MMA issue for the pair ----------------
-        const uint32_t idesc_nv = tc::idesc_fp4(256, 256, 0, 0, 0);
+        // (the whole warp walks the k-steps, one elected lane issues: addresses and descriptors are uniform values)
+        const uint32_t idesc_nv = tc::idesc_fp4(256, 256, 0, 0, 0), tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
         uint32_t g = 0, it = 0;
-        for (int t = pair; t < ntiles && !*abort_flag; t += npairs, it++) {
+        bool ok = true;
+        for (int t = pair; t < ntiles && ok; t += npairs, it++) {
             // the accumulator of the previous tile has been read out by all sixteen epilogue warps of the pair
-            if (it > 0 && !tc::mbar_wait_cluster(accum_empty, (it - 1) & 1u, abort_flag)) {
-                abort_s = 1;
-                atomicExch(p.status, 26);
+            if (it > 0 && !tc::mbar_spin_warp_cluster(accum_empty, (it - 1) & 1u, abort_flag)) {
+                if (lane == 0) {
+                    abort_s = 1;
+                    atomicExch(p.status, 26);
+                }
                 break;
             }
             tc::fence_after_sync();
-            bool ok = true;
             for (int ks = 0; ks < nks; ks++, g++) {
                 const uint32_t s = g % P4_STAGES, ph = (g / P4_STAGES) & 1u;
                 const uint32_t b = g % P4_SF_SETS, bph = (g / P4_SF_SETS) & 1u;
                 // both CTAs' operand tiles have landed, and both CTAs' scale warps have filled column set b
-                if (!tc::mbar_wait(full + 8 * s, ph, abort_flag) || !tc::mbar_wait_cluster(full2 + 8 * s, ph, abort_flag) ||
-                    !tc::mbar_wait_cluster(sf_full + 8 * b, bph, abort_flag)) {
-                    abort_s = 1;
-                    atomicExch(p.status, 22);
+                if (!tc::mbar_spin_warp(full + 8 * s, ph, abort_flag) || !tc::mbar_spin_warp_cluster(full2 + 8 * s, ph, abort_flag) ||
+                    !tc::mbar_spin_warp_cluster(sf_full + 8 * b, bph, abort_flag)) {
+                    if (lane == 0) {
+                        abort_s = 1;
+                        atomicExch(p.status, 22);
+                    }
                     ok = false;
                     break;
                 }
                 tc::fence_after_sync();
                 const uint32_t st = smem_s + s * P4_STAGE_BYTES;
                 const uint64_t ad = tc::smem_desc_sw128(st), bd = tc::smem_desc_sw128(st + P4_A_BYTES);
-                const uint32_t tsfa = tmem + P4_TMEM_SF + P4_SF_SET_COLS * b, tsfb = tsfa + 16;
-                if (p.nv) {
+                const uint32_t tsfa = tmem_u + P4_TMEM_SF + P4_SF_SET_COLS * b, tsfb = tsfa + 16;
+                const uint32_t empty1 = tc::map_to_cta(empty + 8 * s, 1), full1 = tc::map_to_cta(accum_full, 1);
+                if (tc::elect_one()) {
+                    if (p.nv) {
 #pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        tc::mma_nvf4_pair(tmem, ad + 2 * j, bd + 2 * j, idesc_nv, (uint32_t)((ks | j) != 0), tsfa + 4 * j, tsfb + 8 * j);
-                } else {
+                        for (int j = 0; j < 4; j++)
+                            tc::mma_nvf4_pair(tmem_u, ad + 2 * j, bd + 2 * j, idesc_nv, (uint32_t)((ks | j) != 0), tsfa + 4 * j, tsfb + 8 * j);
+                    } else {
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int id = (j & 1) * 2;
-                        tc::mma_mxf4_pair(tmem, ad + 2 * j, bd + 2 * j, tc::idesc_fp4(256, 256, 1, id, id), (uint32_t)((ks | j) != 0),
-                                          tsfa + 4 * (j >> 1), tsfb + 8 * (j >> 1));
+                        for (int j = 0; j < 4; j++) {
+                            const int id = (j & 1) * 2;
+                            tc::mma_mxf4_pair(tmem_u, ad + 2 * j, bd + 2 * j, tc::idesc_fp4(256, 256, 1, id, id), (uint32_t)((ks | j) != 0),
+                                              tsfa + 4 * (j >> 1), tsfb + 8 * (j >> 1));
+                        }
+                    }
+                    // once these MMAs have completed, stage s and column set b are free in BOTH CTAs
+                    tc::mma_commit_pair(empty + 8 * s);
+                    tc::mma_commit_pair(empty1);
+                    if (ks == nks - 1) {
+                        tc::mma_commit_pair(accum_full);
+                        tc::mma_commit_pair(full1);
                     }
                 }
-                // once these MMAs have completed, stage s and column set b are free in BOTH CTAs
-                tc::mma_commit_pair(empty + 8 * s);
-                tc::mma_commit_pair(tc::map_to_cta(empty + 8 * s, 1));
+                __syncwarp();
             }
-            if (!ok) break;
-            tc::mma_commit_pair(accum_full);
-            tc::mma_commit_pair(tc::map_to_cta(accum_full, 1));
         }
     } else if (warp >= 2 + P4_EPI_WARPS) {
         // ---------------- scale warps: stage -> tensor memory, lane quadrant warp % 4 ----------------

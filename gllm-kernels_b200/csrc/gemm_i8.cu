@@ -207,29 +207,33 @@ __global__ void __launch_bounds__(I8_THREADS, 1) gemm_i8_kernel(const __grid_con
             for (int h = 0; h < halves; h++)
                 i8_bulk(st + MT * I8_TILE + h * I8_TILE, p.xt + ((size_t)((tok0 >> 7) + h) * p.nks + ks) * I8_TILE, hb[h], full + 8 * s);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // ---------------- MMA issue: weights signed (operand A), activations unsigned (operand B) ----------------
-        const uint32_t idesc = tc::idesc_i8(I8_BM, ntok, 1, 0);
-        bool ok = true;
+        // (the whole warp walks the k-steps, one elected lane issues: addresses and descriptors are uniform values)
+        const uint32_t idesc = tc::idesc_i8(I8_BM, ntok, 1, 0), tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
         for (int ks = 0; ks < p.nks; ks++) {
             const int s = ks % I8_STAGES;
-            if (!tc::mbar_wait(full + 8 * s, (uint32_t)((ks / I8_STAGES) & 1), abort_flag)) {
-                abort_s = 1;
-                atomicExch(p.status, 42);
-                ok = false;
+            if (!tc::mbar_spin_warp(full + 8 * s, (uint32_t)((ks / I8_STAGES) & 1), abort_flag)) {
+                if (lane == 0) {
+                    abort_s = 1;
+                    atomicExch(p.status, 42);
+                }
                 break;
             }
             tc::fence_after_sync();
             const uint32_t st = smem_s + s * I8_STAGE_BYTES;
             const uint64_t bd = tc::smem_desc_sw128(st + MT * I8_TILE);
-            for (int i = 0; i < mt; i++) {
-                const uint64_t ad = tc::smem_desc_sw128(st + i * I8_TILE);
+            if (tc::elect_one()) {
+                for (int i = 0; i < mt; i++) {
+                    const uint64_t ad = tc::smem_desc_sw128(st + i * I8_TILE);
 #pragma unroll
-                for (int j = 0; j < 4; j++) tc::mma_i8(tmem + 256u * (uint32_t)i, ad + 2 * j, bd + 2 * j, idesc, (uint32_t)((ks | j) != 0));
+                    for (int j = 0; j < 4; j++) tc::mma_i8(tmem_u + 256u * (uint32_t)i, ad + 2 * j, bd + 2 * j, idesc, (uint32_t)((ks | j) != 0));
+                }
+                tc::mma_commit(empty + 8 * s);
+                if (ks == p.nks - 1) tc::mma_commit(accum);
             }
-            tc::mma_commit(empty + 8 * s);
+            __syncwarp();
         }
-        if (ok) tc::mma_commit(accum);
     }
     __syncwarp();
 
@@ -359,41 +363,52 @@ gemm_i8_pair_kernel(const __grid_constant__ I8Params p, const int tok_tiles, con
                 // the stage's bytes are in place before this arrive is issued (the barrier phase was observed)
                 tc::mbar_arrive_cluster_relaxed(tc::map_to_cta(full2 + 8 * s, 0));
             }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && rank == 0) {
         // ---------------- leader CTA: MMA issue for the pair, accumulator (tile & 1) ----------------
+        // (the whole warp walks the k-steps, one elected lane issues: addresses and descriptors are uniform values)
         const uint32_t idesc = tc::idesc_i8(256, I8_BN, 1, 0);  // weights signed (operand A), activations unsigned (operand B)
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
         uint32_t g = 0, it = 0;
-        for (int t = pair; t < ntiles && !*abort_flag; t += npairs, it++) {
+        bool ok = true;
+        for (int t = pair; t < ntiles && ok; t += npairs, it++) {
             const uint32_t acc = it & 1u;
             // the tile before last used this accumulator: all sixteen epilogue warps of the pair have read it out
-            if (it >= 2 && !tc::mbar_wait_cluster(accum_empty + 8 * acc, ((it >> 1) - 1) & 1u, abort_flag)) {
-                abort_s = 1;
-                atomicExch(p.status, 46);
+            if (it >= 2 && !tc::mbar_spin_warp_cluster(accum_empty + 8 * acc, ((it >> 1) - 1) & 1u, abort_flag)) {
+                if (lane == 0) {
+                    abort_s = 1;
+                    atomicExch(p.status, 46);
+                }
                 break;
             }
             tc::fence_after_sync();
-            const uint32_t td = tmem + 256u * acc;
-            bool ok = true;
+            const uint32_t td = tmem_u + 256u * acc;
             for (int ks = 0; ks < p.nks; ks++, g++) {
                 const uint32_t s = g % I8P_STAGES, ph = (g / I8P_STAGES) & 1u;
-                if (!tc::mbar_wait(full + 8 * s, ph, abort_flag) || !tc::mbar_wait_cluster(full2 + 8 * s, ph, abort_flag)) {
-                    abort_s = 1;
-                    atomicExch(p.status, 42);
+                if (!tc::mbar_spin_warp(full + 8 * s, ph, abort_flag) || !tc::mbar_spin_warp_cluster(full2 + 8 * s, ph, abort_flag)) {
+                    if (lane == 0) {
+                        abort_s = 1;
+                        atomicExch(p.status, 42);
+                    }
                     ok = false;
                     break;
                 }
                 tc::fence_after_sync();
                 const uint32_t st = smem_s + s * I8P_STAGE_BYTES;
                 const uint64_t ad = tc::smem_desc_sw128(st), bd = tc::smem_desc_sw128(st + I8_TILE);
+                const uint32_t empty1 = tc::map_to_cta(empty + 8 * s, 1), full1 = tc::map_to_cta(accum_full + 8 * acc, 1);
+                if (tc::elect_one()) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) tc::mma_i8_pair(td, ad + 2 * j, bd + 2 * j, idesc, (uint32_t)((ks | j) != 0));
-                // once these MMAs have completed, stage s is free in BOTH CTAs
-                tc::mma_commit_pair(empty + 8 * s);
-                tc::mma_commit_pair(tc::map_to_cta(empty + 8 * s, 1));
+                    for (int j = 0; j < 4; j++) tc::mma_i8_pair(td, ad + 2 * j, bd + 2 * j, idesc, (uint32_t)((ks | j) != 0));
+                    // once these MMAs have completed, stage s is free in BOTH CTAs
+                    tc::mma_commit_pair(empty + 8 * s);
+                    tc::mma_commit_pair(empty1);
+                    if (ks == p.nks - 1) {
+                        tc::mma_commit_pair(accum_full + 8 * acc);
+                        tc::mma_commit_pair(full1);
+                    }
+                }
+                __syncwarp();
             }
-            if (!ok) break;
-            tc::mma_commit_pair(accum_full + 8 * acc);
-            tc::mma_commit_pair(tc::map_to_cta(accum_full + 8 * acc, 1));
         }
     }
     __syncwarp();

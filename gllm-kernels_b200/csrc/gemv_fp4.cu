@@ -312,57 +312,63 @@ __global__ void __launch_bounds__(FD_THREADS, 1) gemv_fp4_tc_kernel(const __grid
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ---------------- MMA issue ----------------
-            // The scale factors are put into tensor memory by the scale warps (below), not by tcgen05.cp from this thread:
-            // a copy occupies the tensor pipe for ~120 cycles here, eight of them per k-step (NVFP4) were more than half of
-            // the k-step and held the kernel at 0.46 of the HBM bandwidth (MXFP4, four copies: 0.62).
-            int slot = 0, round = 0, seg = 0;
-            uint32_t g = 0;  // k-steps issued by this CTA so far
-            bool ok = true;
-            for (int64_t u = u_begin; u < u_end && ok; seg++) {
-                const int tile = (int)(u / p.nks), j0 = (int)(u - (int64_t)tile * p.nks);
-                const int j1 = (int)min((int64_t)p.nks, (int64_t)j0 + (u_end - u));
-                // the accumulator is rewritten from the segment's first MMA on: the previous epilogue must be done
-                if (seg > 0 && !tc::mbar_wait(tmem_free, (uint32_t)((seg - 1) & 1), abort_flag)) ok = false;
+        // ---------------- MMA issue ----------------
+        // The whole warp walks the k-steps and one elected lane issues: addresses and descriptors are uniform values (with a single
+        // active lane W[8192, 28672], one token, took 35.5 us NVFP4 / 32.3 MXFP4, now 33.1 / 29.5).
+        // The scale factors are put into tensor memory by the scale warps (below), not by tcgen05.cp from this thread:
+        // a copy occupies the tensor pipe for ~120 cycles here, eight of them per k-step (NVFP4) were more than half of
+        // the k-step and held the kernel at 0.46 of the HBM bandwidth (MXFP4, four copies: 0.62).
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+        int slot = 0, round = 0, seg = 0;
+        uint32_t g = 0;  // k-steps issued by this CTA so far
+        bool ok = true;
+        for (int64_t u = u_begin; u < u_end && ok; seg++) {
+            const int tile = (int)(u / p.nks), j0 = (int)(u - (int64_t)tile * p.nks);
+            const int j1 = (int)min((int64_t)p.nks, (int64_t)j0 + (u_end - u));
+            // the accumulator is rewritten from the segment's first MMA on: the previous epilogue must be done
+            if (seg > 0 && !tc::mbar_spin_warp(tmem_free, (uint32_t)((seg - 1) & 1), abort_flag)) ok = false;
+            tc::fence_after_sync();
+            for (int ks = j0; ks < j1 && ok; ks++, g++) {
+                const uint32_t b = g % FD_SF_SETS;
+                if (!tc::mbar_spin_warp(full + 8 * slot, (uint32_t)(round & 1), abort_flag) ||
+                    !tc::mbar_spin_warp(sf_full + 8 * b, (g / FD_SF_SETS) & 1u, abort_flag)) {
+                    ok = false;
+                    break;
+                }
                 tc::fence_after_sync();
-                for (int ks = j0; ks < j1 && ok; ks++, g++) {
-                    const uint32_t b = g % FD_SF_SETS;
-                    if (!tc::mbar_wait(full + 8 * slot, (uint32_t)(round & 1), abort_flag) ||
-                        !tc::mbar_wait(sf_full + 8 * b, (g / FD_SF_SETS) & 1u, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    tc::fence_after_sync();
-                    const uint32_t st = smem_s + (uint32_t)(slot * p.stage_bytes);
-                    const uint64_t ad = tc::smem_desc_sw128(st), bd = tc::smem_desc_sw128(st + b_off);
-                    const uint32_t tsfa = tmem + 128u + 32u * b, tsfb = tsfa + 16u;
-                    const uint32_t first = (uint32_t)(ks != j0);
+                const uint32_t st = smem_s + (uint32_t)(slot * p.stage_bytes);
+                const uint64_t ad = tc::smem_desc_sw128(st), bd = tc::smem_desc_sw128(st + b_off);
+                const uint32_t tsfa = tmem_u + 128u + 32u * b, tsfb = tsfa + 16u;
+                const uint32_t first = (uint32_t)(ks != j0);
+                if (tc::elect_one()) {
                     if (p.nv) {
                         const uint32_t idesc = tc::idesc_fp4(128, p.ncol, 0, 0, 0);
 #pragma unroll
                         for (int j = 0; j < 4; j++)
-                            tc::mma_nvf4(tmem, ad + 2 * j, bd + 2 * j, idesc, first | (uint32_t)(j != 0), tsfa + 4 * j, tsfb + 4 * j);
+                            tc::mma_nvf4(tmem_u, ad + 2 * j, bd + 2 * j, idesc, first | (uint32_t)(j != 0), tsfa + 4 * j, tsfb + 4 * j);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 4; j++) {
                             const int id = (j & 1) * 2;
-                            tc::mma_mxf4(tmem, ad + 2 * j, bd + 2 * j, tc::idesc_fp4(128, p.ncol, 1, id, id), first | (uint32_t)(j != 0),
+                            tc::mma_mxf4(tmem_u, ad + 2 * j, bd + 2 * j, tc::idesc_fp4(128, p.ncol, 1, id, id), first | (uint32_t)(j != 0),
                                          tsfa + 4 * (j >> 1), tsfb + 4 * (j >> 1));
                         }
                     }
                     tc::mma_commit(empty + 8 * slot);
                     tc::mma_commit(sf_empty + 8 * b);
-                    if (++slot == p.stages) slot = 0, round++;
+                    if (ks == j1 - 1) tc::mma_commit(accum);
                 }
-                if (!ok) {
+                __syncwarp();
+                if (++slot == p.stages) slot = 0, round++;
+            }
+            if (!ok) {
+                if (lane == 0) {
                     abort_s = 1;
                     atomicExch(p.status, 52);
-                    break;
                 }
-                tc::mma_commit(accum);
-                u += j1 - j0;
+                break;
             }
+            u += j1 - j0;
         }
     } else if (warp >= 6) {
         // ---------------- scale warps: stage -> tensor memory, lane quadrant warp % 4 ----------------

@@ -264,6 +264,23 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
     }
     return false;
 }
+// back-to-back probes by a whole warp that stays together (mbar_spin_warp), acquiring arrivals from the other CTA as well
+__device__ __forceinline__ bool mbar_spin_warp_cluster(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+#pragma unroll 1
+    for (uint32_t it = 0; it < (1u << 22); it++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n.reg .pred p;\n"
+            "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (__all_sync(0xffffffffu, (int)ok)) return true;
+        if ((it & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag)) return false;
+    }
+    return false;
+}
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 // TMEM of both CTAs of the pair: the same warp of BOTH CTAs executes these, with the same operands
