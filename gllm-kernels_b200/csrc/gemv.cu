@@ -76,14 +76,24 @@ __global__ void __launch_bounds__(256) stage_x_kernel(StageParams p) {
     const int64_t k0 = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 4;
     const float *xr = p.x + (int64_t)tok * p.xst;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (k0 < p.K) {
+    // contiguous rows: one 16-byte load (x may lie in page-locked host memory, where every load is a transfer over PCIe)
+    const auto load4 = [&](const float *row, float (&o)[4]) {
+        if (p.xsk == 1 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+            const float4 q = *reinterpret_cast<const float4 *>(row + k0);
+            o[0] = q.x, o[1] = q.y, o[2] = q.z, o[3] = q.w;
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = xr[(k0 + i) * p.xsk];
+            for (int i = 0; i < 4; i++) o[i] = row[(k0 + i) * p.xsk];
+        }
+    };
+    if (k0 < p.K) {  // K is a multiple of 32: all four elements exist
+        load4(xr, v);
         if (p.x_up) {
             // swiglu (scalar-ops/src/activations.rs:57-66): out = g / (1 + exp(-g)) * u, in f32
-            const float *ur = p.x_up + (int64_t)tok * p.xst;
+            float u[4];
+            load4(p.x_up + (int64_t)tok * p.xst, u);
 #pragma unroll
-            for (int i = 0; i < 4; i++) v[i] = (v[i] / (1.0f + expf(-v[i]))) * ur[(k0 + i) * p.xsk];
+            for (int i = 0; i < 4; i++) v[i] = (v[i] / (1.0f + expf(-v[i]))) * u[i];
         }
     }
     float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));

@@ -57,8 +57,13 @@ __global__ void __launch_bounds__(256) raw_mma_stage_kernel(const RmStage p) {
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     if (k0 < p.k) {
         const float *xr = p.x + (int64_t)tok * p.xst + k0 * p.xsk;
+        if (p.xsk == 1 && (reinterpret_cast<uintptr_t>(xr) & 15) == 0) {
+            const float4 q = *reinterpret_cast<const float4 *>(xr);
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = xr[i * p.xsk];
+            for (int i = 0; i < 4; i++) v[i] = xr[i * p.xsk];
+        }
     }
     float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
     const float inf = __int_as_float(0x7F800000);

@@ -36,10 +36,26 @@ def _ptr(a) -> int:
     return a.data_ptr()
 
 
+_current_raw_stream = None
+
+
+def _find_raw_stream():
+    """The handle of the current stream without building a Stream object for it (3.2 us of a 16 us decode call): torch's own
+    accessors where this torch has them."""
+    import torch
+    c = torch._C
+    if hasattr(c, "_cuda_getCurrentRawStream") and hasattr(c, "_cuda_getDevice"):
+        torch.cuda.current_stream()  # initialises CUDA as the public call would
+        return lambda: c._cuda_getCurrentRawStream(c._cuda_getDevice())
+    return lambda: torch.cuda.current_stream().cuda_stream
+
+
 def _stream(stream) -> int:
+    global _current_raw_stream
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        if _current_raw_stream is None:
+            _current_raw_stream = _find_raw_stream()
+        return _current_raw_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
