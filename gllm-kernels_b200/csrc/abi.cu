@@ -844,7 +844,7 @@ static int32_t matmul_host_impl(Ctx *c, const Weight *w, const float *x_host, in
     if (sb) GK_CUDA(c, cudaMemcpyAsync(dev + so, pin + so, sb, cudaMemcpyHostToDevice, c->stream));
     const float *xd = reinterpret_cast<const float *>(zero_copy_x ? static_cast<const char *>(x_alias) : dev + xo);
     // The decode kernels' stores go straight to a page-locked result, beside the products that are still running; the context's
-    // own page-locked area serves the others the same way (W[11008, 4096]: Q8_0 x 8 tokens 54 -> 50 us per call, Q6_K 54 -> 47, one token
+    // own page-locked area serves the others the same way (W[11008, 4096]: Q8_0 x 8 tokens 54 -> 43 us per call, Q6_K 54 -> 46, one token
     // 34 -> 31; a 0.9 MB result is better copied, 65 against 68 us).  A token's rows lie side by side.
     const bool decode = ref_layout || sb || m_t <= GLLMK_GEMM_GEMV_MAX_M || raw_format(w->qt);
     const bool zero_copy_y = decode && m_t <= GLLMK_GEMV_MAX_M && (!ref_layout || m_t == 1) && yb <= (size_t)512 * 1024;

@@ -45,15 +45,15 @@ struct RmStage {
     uint8_t *img;
 };
 
-// Thread = four elements; 64 threads = one 256-element block.  In a run, elements 4t .. 4t + 3 and 16 + 4t .. + 3 are lane t's two
+// Thread = four elements; a CTA's 64 threads = one 256-element block.  In a run, elements 4t .. 4t + 3 and 16 + 4t .. + 3 are lane t's two
 // operand-B words (byte 8t of the run).
-__global__ void __launch_bounds__(256) raw_mma_stage_kernel(const RmStage p) {
-    __shared__ float wmax[8];
-    __shared__ int wbad[8];
+__global__ void __launch_bounds__(64) raw_mma_stage_kernel(const RmStage p) {
+    __shared__ float wmax[2];
+    __shared__ int wbad[2];
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     const int tok = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t k0 = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 4;  // k is a multiple of 256: a block is inside or outside as a whole
+    const int64_t k0 = ((int64_t)blockIdx.x * 64 + threadIdx.x) * 4;  // k is a multiple of 256: a block is inside or outside as a whole
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     if (k0 < p.k) {
         const float *xr = p.x + (int64_t)tok * p.xst + k0 * p.xsk;
@@ -757,7 +757,7 @@ int32_t raw_mma_launch(Ctx *c, const Weight *w, const float *x, int64_t xst, int
         p.m = m - t0 < RM_PASS ? m - t0 : RM_PASS;
         p.y = y + (int64_t)t0 * yst;
         RmStage sp{x + (int64_t)t0 * xst, xst, xsk, w->k, p.m, w->qt == GLLMK_QUANT_Q5_K, static_cast<uint8_t *>(c->act)};
-        GK_CUDA(c, launch_after(raw_mma_stage_kernel, dim3((unsigned)((w->k + 1023) / 1024), (unsigned)p.m), 256, 0, s, sp));
+        GK_CUDA(c, launch_after(raw_mma_stage_kernel, dim3((unsigned)nb, (unsigned)p.m), 64, 0, s, sp));
         switch (w->qt) {
             case GLLMK_QUANT_Q6_K: rc = rm_format<GLLMK_QUANT_Q6_K>(c, p, s); break;
             case GLLMK_QUANT_Q5_K: rc = rm_format<GLLMK_QUANT_Q5_K>(c, p, s); break;
