@@ -86,7 +86,7 @@ struct GemmParams {
     int y_bf16;
     int64_t ldy;
     int vec;             // Y allows 16-byte stores
-    int ntok, ntok32;    // MMA N of this launch (multiple of 16; <= 192 with two row tiles, <= 256 with one); rounded up to 32
+    int ntok, ntok32;    // largest MMA N of this launch (multiple of 16; <= 192 with two row tiles, <= 256 with one); rounded up to 32
     int row_tiles;       // 128-row tiles of the weight matrix
     int sb, r;           // ring depths: B stages, raw super-chunks
     int *status;
@@ -551,6 +551,8 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
     const int mt = min(MT, p.row_tiles - tile0);  // row tiles this CTA really has
     const int grp_id = G.tile_group[bx];
     const int64_t tok0 = G.tile_tok0[bx], tok_end = tok0 + G.tile_cnt[bx];
+    // the MMA's N is this tile's own token count (a multiple of 16): the last tile of a batch and the experts of a layer differ
+    const int ntile = min(p.ntok, (G.tile_cnt[bx] + 15) & ~15), ntile32 = (ntile + 31) & ~31;
     const int nks = 4 * njb, nks_row = 4 * p.nsc;  // k-steps of this unit / of a whole row
     volatile int *abort_flag = &abort_s;
 
@@ -653,9 +655,9 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
     } else if (warp == 1) {
         // ---------------- activation tiles: one thread, bulk copies ----------------
         if (lane == 0) {
-            // a tile of more than 128 tokens is two activation images: a whole one and the first ntok - 128 rows
-            const int halves = (p.ntok + 127) / 128, img0 = G.tile_img[bx];
-            const uint32_t hbytes[2] = {(uint32_t)(p.ntok > 128 ? WQ_TILE : bstage), (uint32_t)(bstage - WQ_TILE)};
+            // a tile of more than 128 tokens is two activation images: a whole one and the first ntile - 128 rows
+            const int halves = (ntile + 127) / 128, img0 = G.tile_img[bx];
+            const uint32_t hbytes[2] = {(uint32_t)(ntile > 128 ? WQ_TILE : ntile * 128), (uint32_t)(ntile * 128 - WQ_TILE)};
             int slot = 0, round = 0;
             asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the staging kernel's tile images are complete from here on
             for (int ks = 0; ks < nks; ks++) {
@@ -667,7 +669,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
                 }
                 WQP_ACC(0);
                 const uint32_t dst = smem_s + b_off + (uint32_t)(slot * bstage);
-                tc::mbar_expect_tx(fullB + 8 * slot, (uint32_t)bstage);
+                tc::mbar_expect_tx(fullB + 8 * slot, (uint32_t)(ntile * 128));
                 for (int h = 0; h < halves; h++)
                     bulk_g2s(dst + h * WQ_TILE, p.xt + ((size_t)(img0 + h) * nks_row + 4 * jb0 + ks) * WQ_TILE, hbytes[h], fullB + 8 * slot);
                 if (++slot == p.sb) slot = 0, round++;
@@ -682,7 +684,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
         const int i = __shfl_sync(0xffffffffu, warp, 0) - 2;
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_d, 0);
         if (i < mt) {
-            const uint32_t idesc = tc::idesc_f16(WQ_BM, p.ntok, 0, 0);  // fp16 x fp16 -> f32
+            const uint32_t idesc = tc::idesc_f16(WQ_BM, ntile, 0, 0);  // fp16 x fp16 -> f32
             bool ok = true;
             int sb = 0, bround = 0;
             for (int ks = 0; ks < nks; ks++) {
@@ -789,7 +791,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
             if (nsplit == 1) {
                 for (int i = 0; i < mt; i++) {
                     const int64_t row_base = (int64_t)(tile0 + i) * WQ_BM + 32 * quad;
-                    for (int c = 32 * (dw >> 2); c < p.ntok32; c += 32 * (WQ_DW / 4)) {
+                    for (int c = 32 * (dw >> 2); c < ntile32; c += 32 * (WQ_DW / 4)) {
                         uint32_t v[32];
                         tc::tmem_ld32(tmem_d + ((uint32_t)(32 * quad) << 16) + WQ_ACC2 * (uint32_t)i + (uint32_t)c, v);
                         tc::tmem_ld_wait();
@@ -807,7 +809,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
                 const size_t unit_floats = (size_t)MT * p.ntok32 * WQ_BM;
                 float *tile_part = p.partial + (size_t)tail_tile * nsplit * unit_floats, *mine = tile_part + (size_t)split * unit_floats;
                 for (int i = 0; i < mt; i++)
-                    for (int c = 32 * (dw >> 2); c < p.ntok32; c += 32 * (WQ_DW / 4)) {
+                    for (int c = 32 * (dw >> 2); c < ntile32; c += 32 * (WQ_DW / 4)) {
                         uint32_t v[32];
                         tc::tmem_ld32(tmem_d + ((uint32_t)(32 * quad) << 16) + WQ_ACC2 * (uint32_t)i + (uint32_t)c, v);
                         tc::tmem_ld_wait();
@@ -828,7 +830,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
                 if (last_s) {
                     for (int i = 0; i < mt; i++) {
                         const int64_t row_base = (int64_t)(tile0 + i) * WQ_BM + 32 * quad;
-                        for (int c = 32 * (dw >> 2); c < p.ntok32; c += 32 * (WQ_DW / 4)) {
+                        for (int c = 32 * (dw >> 2); c < ntile32; c += 32 * (WQ_DW / 4)) {
                             float o[32];
 #pragma unroll
                             for (int jj = 0; jj < 32; jj++) o[jj] = 0.0f;
