@@ -463,3 +463,47 @@ def test_fp4_activations_uploaded_per_call_reuse_freed_buffers(gk, K, ms):
     assert K.status() == 0
     for a, b in zip(got, ref):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("fmt", ["q4k", "mxfp4"])
+@pytest.mark.parametrize("row_tiles", [1, 2])
+@pytest.mark.parametrize("m", [17, 127, 128, 129, 176, 192, 193, 208, 256, 257, 400])
+def test_gemm_token_tiles_around_the_accumulators_sizes(gk, K, oracle, fmt, row_tiles, m):
+    """Weight tiles in tensor memory beside one or two accumulators: token counts at the edges of the tile sizes (16, 128, 192 for
+    two row tiles, 256), one format per store form (thread = row; quads).  Both operands are rounded to fp16 (2^-11 each) and a
+    Q4_K weight once more after its product: 3 x 2^-11 = 1.5e-3 at most in the norm, sums in f32."""
+    import torch
+    n, k = 512, 768
+    qt, blocks, scales, g, wd = quantized(oracle, gk, fmt, n, k, 40 + m)
+    w = K.upload(qt, n, k, blocks, scales, g)
+    x = np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)
+    try:
+        K.set("gemm_row_tiles", row_tiles)
+        y = K.gemm(w, torch.from_numpy(x).cuda()).cpu().numpy()
+    finally:
+        K.set("gemm_row_tiles", 0)
+    want = x.astype(np.float64) @ wd.reshape(n, k).astype(np.float64).T
+    assert K.status() == 0
+    assert np.linalg.norm(y - want) <= 1.5e-3 * np.linalg.norm(want)
+    w.free()
+
+
+@pytest.mark.parametrize("counts", [(0, 1, 193, 70, 256, 33), (16, 17, 0, 0, 400, 1), (5, 5, 5, 5, 5, 5)])
+def test_gemm_grouped_tiles_of_their_own_token_counts(gk, K, oracle, counts):
+    """Experts whose token counts differ widely: every tile's MMA takes its own count, rounded up to 16 (bound as above)."""
+    import torch
+    n, k = 384, 512
+    rng = np.random.default_rng(sum(counts))
+    offs = np.concatenate(([0], np.cumsum(counts)))
+    x = rng.standard_normal((int(offs[-1]), k)).astype(np.float32)
+    parts = [quantized(oracle, gk, "q8_0", n, k, 60 + e) for e in range(len(counts))]
+    ws = [K.upload(qt, n, k, b, s, g) for qt, b, s, g, _ in parts]
+    y = K.gemm_grouped(ws, torch.from_numpy(x).cuda(), [int(o) for o in offs]).cpu().numpy()
+    assert K.status() == 0
+    for e, (_, _, _, _, wd) in enumerate(parts):
+        lo, hi = int(offs[e]), int(offs[e + 1])
+        if hi > lo:
+            want = x[lo:hi].astype(np.float64) @ wd.reshape(n, k).astype(np.float64).T
+            assert np.linalg.norm(y[lo:hi] - want) <= 1.5e-3 * np.linalg.norm(want), e
+    for w in ws:
+        w.free()

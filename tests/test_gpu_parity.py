@@ -566,3 +566,18 @@ def test_fp4_quantizers_ties_clamps_and_alignment(gk, K, oracle, torch, fmt, n, 
         rb, rg = oracle.quantize_nvfp4(W, global_scale) if global_scale else oracle.quantize_nvfp4(W)
         assert g == pytest.approx(rg, rel=0, abs=0)
         assert np.array_equal(b.cpu().numpy(), rb)
+
+
+@pytest.mark.parametrize("n,m", [(1000, 1), (1000, 8), (513, 16), (20000, 8)])
+@pytest.mark.parametrize("pinned", [True, False])
+def test_matmul_host_results_up_to_half_a_megabyte_are_stored_directly(gk, K, oracle, torch, n, m, pinned):
+    """Small results go straight to page-locked memory (the caller's or the context's own), larger ones are copied: both are what
+    the device call gives, bit for bit."""
+    k = 512
+    w = K.upload(gk.QuantType.q8_0(), n, k, oracle.quantize_q8_0((np.random.default_rng(n).standard_normal((n, k)) * 0.02).astype(np.float32)))
+    x = np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)
+    out = torch.full((m, n), float("nan"), pin_memory=pinned).numpy()
+    K.matmul_host(w, x, out=out)
+    assert np.array_equal(out, K.gemv(w, torch.from_numpy(x).cuda()).cpu().numpy())
+    assert K.status() == 0
+    w.free()
