@@ -109,8 +109,11 @@ __global__ void __launch_bounds__(256) stage_act_kernel(const void *__restrict__
     // The GEMM behind this launch may start now (programmatic dependent launch): its CTAs take the SMs this grid leaves,
     // allocate tensor memory and stream raw weights; the one thread that reads these tile images orders itself after
     // this grid with griddepcontrol.wait.
+    // This grid is itself launched early: it reads a and overwrites the images once everything in front of it has completed.
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     const int ks = blockIdx.x, tile = blockIdx.y;
+    // (loads through L2: a may be the output of the grid this one was launched behind)
     const int64_t img_tok0 = imgs.tok0[tile];
     const int img_cnt = imgs.cnt[tile];
     uint8_t *dst = xt + ((size_t)tile * gridDim.x + ks) * WQ_TILE;
@@ -122,11 +125,11 @@ __global__ void __launch_bounds__(256) stage_act_kernel(const void *__restrict__
         if (row < img_cnt && k0 < k_valid) {
             if (a_bf16) {
                 // bf16 -> fp16 through f32, saturating at +-65504
-                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(a) + tok * lda + k0));
+                const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(a) + tok * lda + k0));
                 const uint32_t w[4] = {v.x, v.y, v.z, v.w};
                 uint32_t r[4];
                 if (a_up) {
-                    const uint4 vu = __ldg(reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(a_up) + tok * lda + k0));
+                    const uint4 vu = __ldcg(reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(a_up) + tok * lda + k0));
                     const uint32_t wu[4] = {vu.x, vu.y, vu.z, vu.w};
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
@@ -142,10 +145,10 @@ __global__ void __launch_bounds__(256) stage_act_kernel(const void *__restrict__
                 o = make_uint4(r[0], r[1], r[2], r[3]);
             } else {
                 const float4 *src = reinterpret_cast<const float4 *>(static_cast<const float *>(a) + tok * lda + k0);
-                float4 x0 = __ldg(src), x1 = __ldg(src + 1);
+                float4 x0 = __ldcg(src), x1 = __ldcg(src + 1);
                 if (a_up) {
                     const float4 *su = reinterpret_cast<const float4 *>(static_cast<const float *>(a_up) + tok * lda + k0);
-                    const float4 u0 = __ldg(su), u1 = __ldg(su + 1);
+                    const float4 u0 = __ldcg(su), u1 = __ldcg(su + 1);
                     x0 = make_float4(swiglu_f32(x0.x, u0.x), swiglu_f32(x0.y, u0.y), swiglu_f32(x0.z, u0.z), swiglu_f32(x0.w, u0.w));
                     x1 = make_float4(swiglu_f32(x1.x, u1.x), swiglu_f32(x1.y, u1.y), swiglu_f32(x1.z, u1.z), swiglu_f32(x1.w, u1.w));
                 }
@@ -533,6 +536,9 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
                    emptyB = fullB + 8 * WQ_MAX_SB, rawfull = emptyB + 8 * WQ_MAX_SB, rawempty = rawfull + 8 * WQ_MAX_R,
                    accum = rawempty + 8 * WQ_MAX_R;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // The next call's staging kernel and, behind it, its GEMM may take the SMs this grid leaves: the staging kernel waits for this
+    // grid, and nothing of the GEMM but its weight copies runs ahead of the staging kernel.
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     // which tile, and which part of its k range
     int bx = blockIdx.x, by = blockIdx.y, jb0 = 0, njb = p.nsc, split = 0, nsplit = 1, tail_tile = 0;
     if (p.split_s > 1) {
@@ -575,6 +581,55 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
         tc::mbar_init(accum, (uint32_t)mt);
         tc::mbar_init_fence();
     }
+    // ---------------- raw weight super-chunks ----------------
+    // Super-chunk q: k-block jb0 + q / mt, row tile q % mt of the CTA.  Q4_K / Q8_0: the eight 16-row chunks of a 128-row tile for a
+    // k-block are contiguous, one bulk copy; FP4: a tile image and its scale atoms.  The blocks of a row-major tile lie a whole row
+    // apart in memory, 128 pieces of 224 / 176 / 144 bytes: as 128 bulk copies they paced the kernel (a copy engine request per
+    // piece: ~1.8 k cycles per tile step); the whole warp copies them with 16-byte cp.async instead — 64 per lane, half a warp per
+    // row piece (lane % 16 = 16-byte chunk, the lanes past the piece's chunks idle; rows 2 j + lane / 16), so that an iteration is
+    // the copy and two additions — and every lane's copies arrive at the slot's barrier when they have landed
+    // (cp.async.mbarrier.arrive.noinc).
+    const auto copy_raw = [&](int q, int slot) {
+        const int jb = jb0 + (mt == 2 ? q >> 1 : q), tile = tile0 + (mt == 2 ? q & 1 : 0);
+        const uint32_t dst = smem_s + raw_off + (uint32_t)(slot * RAW);
+        if constexpr (wq_row_major(FMT)) {
+            constexpr int SLOT = wq_slot(FMT), RSTRIDE = wq_row_stride(FMT), CPR = SLOT / 16;  // 16-byte chunks per row piece
+            const int64_t trow0 = (int64_t)tile * WQ_BM;
+            const int rmax = (int)(p.n - 1 - trow0 < WQ_BM - 1 ? p.n - 1 - trow0 : WQ_BM - 1);  // rows past the matrix repeat the last one; not stored
+            const size_t row_bytes = (size_t)p.nsc * SLOT;
+            const int hrow = lane >> 4, ch = lane & 15;
+            const uint8_t *tile_src = G.qs[grp_id] + ((size_t)trow0 * p.nsc + jb) * SLOT + 16 * ch;
+            if (ch < CPR) {
+                if (rmax == WQ_BM - 1) {
+                    const uint8_t *src = tile_src + (size_t)hrow * row_bytes;
+                    uint32_t d = dst + (uint32_t)(hrow * RSTRIDE + 16 * ch);
+#pragma unroll 8
+                    for (int j = 0; j < WQ_BM / 2; j++, src += 2 * row_bytes, d += 2 * RSTRIDE) cp_async16_s(d, src);
+                } else {
+                    for (int r = hrow; r < WQ_BM; r += 2)
+                        cp_async16_s(dst + (uint32_t)(r * RSTRIDE + 16 * ch), tile_src + (size_t)(r < rmax ? r : rmax) * row_bytes);
+                }
+            }
+            cp_async_arrive(rawfull + 8 * slot);
+        } else {
+            tc::mbar_expect_tx(rawfull + 8 * slot, RAW);
+            if constexpr (FMT == FMT_Q4K || FMT == FMT_Q80) {
+                bulk_g2s(dst, G.qs[grp_id] + ((size_t)tile * p.nsc + jb) * RAW, RAW, rawfull + 8 * slot);
+            } else {
+                constexpr int SFB = RAW - WQ_TILE;
+                bulk_g2s(dst, G.qs[grp_id] + ((size_t)tile * p.nsc + jb) * WQ_TILE, WQ_TILE, rawfull + 8 * slot);
+                bulk_g2s(dst + WQ_TILE, G.aux[grp_id] + ((size_t)tile * p.nsc + jb) * SFB, SFB, rawfull + 8 * slot);
+            }
+        }
+    };
+    const int nraw = njb * mt, raw_pre = min(nraw, p.r);
+    // the first ring-full needs nothing but the barriers: under way before tensor memory is allocated
+    if (warp == 0) {
+        __syncwarp();
+        if (wq_row_major(FMT) || lane == 0)
+            for (int q = 0; q < raw_pre; q++) copy_raw(q, q);
+        __syncwarp();
+    }
     if (warp == 2) tc::tmem_alloc(tc::smem_u32(&tmem_base_s), WQ_TMEM);
     tc::fence_before_sync();
     __syncthreads();
@@ -582,76 +637,24 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
     const uint32_t tmem_d = tmem_base_s;
     WQP_DECL;
 
-    if (warp == 0 && wq_row_major(FMT)) {
-        constexpr int SLOT = wq_slot(FMT), RSTRIDE = wq_row_stride(FMT), CPR = SLOT / 16;  // 16-byte chunks per row piece
-        // ---------------- raw weight blocks: one block of each of the tile's 128 rows per super-chunk ----------------
-        // The blocks of a tile lie a whole row apart in memory, so a super-chunk is 128 pieces of 224 / 176 / 144 bytes.  As 128
-        // bulk copies they paced the kernel (a copy engine request per piece: ~1.8 k cycles per tile step); the whole warp
-        // copies them with 16-byte cp.async instead — 64 per lane — and every lane's copies arrive at the slot's barrier
-        // when they have landed (cp.async.mbarrier.arrive.noinc).
-        int slot = 0, round = 0;
-        bool ok = true;
-        for (int jl = 0; jl < njb && ok; jl++) {
-            const int jb = jb0 + jl;
-            for (int ti = 0; ti < mt && ok; ti++) {
-                if (lane == 0 && round > 0 && !tc::mbar_wait(rawempty + 8 * slot, (uint32_t)((round - 1) & 1), abort_flag)) {
+    if (warp == 0) {
+        // ---------------- raw weight super-chunks, the rest ----------------
+        // (row-major formats: the whole warp copies; the others: one thread's bulk copies)
+        if (wq_row_major(FMT) || lane == 0) {
+            int slot = raw_pre == p.r ? 0 : raw_pre, round = raw_pre == p.r ? 1 : 0;
+            for (int q = raw_pre; q < nraw; q++) {
+                WQP_T0();
+                bool ok = true;
+                if (round > 0 && lane == 0 && !tc::mbar_wait(rawempty + 8 * slot, (uint32_t)((round - 1) & 1), abort_flag)) {
                     abort_s = 1;
                     atomicExch(p.status, 10);
                     ok = false;
                 }
-                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+                if (wq_row_major(FMT)) ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
                 if (!ok) break;
-                const uint32_t dst = smem_s + raw_off + (uint32_t)(slot * RAW);
-                const int64_t trow0 = (int64_t)(tile0 + ti) * WQ_BM;
-                const int rmax = (int)(p.n - 1 - trow0 < WQ_BM - 1 ? p.n - 1 - trow0 : WQ_BM - 1);  // rows past the matrix repeat the last one; not stored
-                // half a warp per row piece: lane % 16 = 16-byte chunk (the lanes past the piece's CPR chunks idle), rows 2 j +
-                // lane / 16 — constant strides, so an iteration is the copy and two additions
-                const size_t row_bytes = (size_t)p.nsc * SLOT;
-                const int hrow = lane >> 4, ch = lane & 15;
-                const uint8_t *tile_src = G.qs[grp_id] + ((size_t)trow0 * p.nsc + jb) * SLOT + 16 * ch;
-                if (ch < CPR) {
-                    if (rmax == WQ_BM - 1) {
-                        const uint8_t *src = tile_src + (size_t)hrow * row_bytes;
-                        uint32_t d = dst + (uint32_t)(hrow * RSTRIDE + 16 * ch);
-#pragma unroll 8
-                        for (int j = 0; j < WQ_BM / 2; j++, src += 2 * row_bytes, d += 2 * RSTRIDE) cp_async16_s(d, src);
-                    } else {
-                        for (int r = hrow; r < WQ_BM; r += 2)
-                            cp_async16_s(dst + (uint32_t)(r * RSTRIDE + 16 * ch), tile_src + (size_t)(r < rmax ? r : rmax) * row_bytes);
-                    }
-                }
-                cp_async_arrive(rawfull + 8 * slot);
+                WQP_ACC(0);
+                copy_raw(q, slot);
                 if (++slot == p.r) slot = 0, round++;
-            }
-        }
-    } else if (warp == 0) {
-        // ---------------- raw weight super-chunks: one thread, bulk copies ----------------
-        if (lane == 0) {
-            int slot = 0, round = 0;
-            for (int jl = 0; jl < njb; jl++) {
-                const int jb = jb0 + jl;
-                for (int ti = 0; ti < mt; ti++) {
-                    WQP_T0();
-                    if (round > 0 && !tc::mbar_wait(rawempty + 8 * slot, (uint32_t)((round - 1) & 1), abort_flag)) {
-                        abort_s = 1;
-                        atomicExch(p.status, 10);
-                        jl = njb;
-                        break;
-                    }
-                    WQP_ACC(0);
-                    const int tile = tile0 + ti;
-                    const uint32_t dst = smem_s + raw_off + (uint32_t)(slot * RAW);
-                    tc::mbar_expect_tx(rawfull + 8 * slot, RAW);
-                    if (FMT == FMT_Q4K || FMT == FMT_Q80) {
-                        // the eight 16-row chunks of a 128-row tile for k-block jb are contiguous
-                        bulk_g2s(dst, G.qs[grp_id] + ((size_t)tile * p.nsc + jb) * RAW, RAW, rawfull + 8 * slot);
-                    } else {
-                        constexpr int SFB = RAW - WQ_TILE;
-                        bulk_g2s(dst, G.qs[grp_id] + ((size_t)tile * p.nsc + jb) * WQ_TILE, WQ_TILE, rawfull + 8 * slot);
-                        bulk_g2s(dst + WQ_TILE, G.aux[grp_id] + ((size_t)tile * p.nsc + jb) * SFB, SFB, rawfull + 8 * slot);
-                    }
-                    if (++slot == p.r) slot = 0, round++;
-                }
             }
         }
     } else if (warp == 1) {
@@ -1007,8 +1010,8 @@ static int32_t gemm_groups_chunk(Ctx *c, const Weight *const *ws, int ng, const 
     int32_t rc = ensure_act(c, (size_t)nimg * nks * WQ_TILE);
     if (rc) return rc;
     p.xt = static_cast<const uint8_t *>(c->act);
-    stage_act_kernel<<<dim3((unsigned)nks, (unsigned)nimg), 256, 0, s>>>(a, a_bf16, lda, w->k, static_cast<uint8_t *>(c->act), imgs, a_up, wq_quads(fmt) ? 1 : 0);
-    GK_CUDA(c, cudaGetLastError());
+    GK_CUDA(c, launch_after(stage_act_kernel, dim3((unsigned)nks, (unsigned)nimg), 256, 0, s, a, a_bf16, lda, (int64_t)w->k,
+                            static_cast<uint8_t *>(c->act), imgs, a_up, wq_quads(fmt) ? 1 : 0));
     dim3 grid((unsigned)ntiles, (unsigned)((row_tiles + mt - 1) / mt));
     // Tail split: the last, partly filled wave of tiles — the only one, when there are fewer tiles than SMs — is cut along
     // k so that its work spreads over all SMs (224 tiles on 148 SMs: 148 whole tiles, then 76 tiles in thirds = 228 units
