@@ -63,21 +63,19 @@ __device__ __forceinline__ uint64_t fd_sf_desc(uint32_t smem_addr) {
 }
 
 // ---- activations -> eight FP4 digit rows per token ---------------------------------------------------------
-// nearest E2M1 code of r (|r| <= 6 up to rounding); residual after it is at most 1 (between 4 and 6)
+// nearest E2M1 code of r (|r| <= 6 up to rounding) and its value, by the hardware conversions there and back (exact ties go to
+// the even code; what is left then has the same size with the other sign); the residual is at most 1 (between 4 and 6).  Eight
+// digits are a chain of eight of these: with a search of the seven thresholds the chain was the staging kernel's longest part.
 __device__ __forceinline__ uint32_t fd_e2m1(float r, float &val) {
-    const float a = fabsf(r);
-    uint32_t c;
-    float v;
-    if (a < 0.25f) c = 0, v = 0.0f;
-    else if (a < 0.75f) c = 1, v = 0.5f;
-    else if (a < 1.25f) c = 2, v = 1.0f;
-    else if (a < 1.75f) c = 3, v = 1.5f;
-    else if (a < 2.5f) c = 4, v = 2.0f;
-    else if (a < 3.5f) c = 5, v = 3.0f;
-    else if (a < 5.0f) c = 6, v = 4.0f;
-    else c = 7, v = 6.0f;
-    val = r < 0.0f ? -v : v;
-    return c | (r < 0.0f ? 8u : 0u);
+    uint32_t c, h;
+    asm("{\n.reg .b8 a, z;\n.reg .b32 t;\nmov.b32 t, 0;\nmov.b32 {z, _, _, _}, t;\n"
+        "cvt.rn.satfinite.e2m1x2.f32 a, 0f00000000, %2;\n"
+        "mov.b32 %0, {a, z, z, z};\n"
+        "cvt.rn.f16x2.e2m1x2 %1, a;\n}\n"
+        : "=r"(c), "=r"(h)
+        : "f"(r));
+    val = __half2float(__ushort_as_half((unsigned short)(h & 0xFFFFu)));
+    return c & 15u;
 }
 // smallest UE4M3 value >= v (0 < v <= 448): code, and its value in `dec`
 __device__ __forceinline__ uint32_t fd_ue4m3_up(float v, float &dec) {
