@@ -699,9 +699,10 @@ int32_t rm_pass(Ctx *c, RmParams &p, cudaStream_t s) {
     if (ctas > units) ctas = units;
     // few units per CTA: no more CTAs than the longest share needs — 512 units on 444 CTAs take as long as on 256 CTAs of two, whose
     // tiles have half the shares to write, count and add up (W[4096, 4096]: 13.1 -> 12.2 us at 5 tokens, W[11008, 4096], four units:
-    // 15.7 -> 14.8).  With one or two tokens and two units the smaller grid is the slower one (10.2 against 10.6 us)
+    // 15.7 -> 14.8).  With one or two tokens and two units, or two units in a few CTAs only, the larger
+    // grid is the faster one (10.2 against 10.6 us)
     const int64_t longest = (units + ctas - 1) / ctas;
-    if (longest <= 4 && (longest > 2 || NG > 1)) ctas = (units + longest - 1) / longest;
+    if (longest <= 4 && (longest > 2 || (NG > 1 && units * 10 >= ctas * 11))) ctas = (units + longest - 1) / longest;
     if (units / ctas > 0x3fffffff) return fail(c, GLLMK_STATUS_INVALID_ARG, "gemv: matrix too large");
     p.per_cta = (int)(units / ctas);
     p.rem = (int)(units % ctas);
