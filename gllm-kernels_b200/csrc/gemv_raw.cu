@@ -19,7 +19,7 @@
 // in brackets the kernels before: dp2a on CUDA cores, and for Q6_K of two tokens and more an MMA kernel of 16 rows per CTA whose
 // warps staged the activations each for themselves:
 //   W[8192, 28672]   1 token            8 tokens     16 tokens         W[11008, 4096], 5 tokens
-//   Q6_K             50 (62)  3.9 TB/s   72 (100)    117 (135)         19
+//   Q6_K             49 (62)  3.9 TB/s   72 (100)    117 (135)         19
 //   Q5_K             44 (73)  3.6 TB/s   61          87 (590)          18 (61)
 //   Q8_K             53 (69)  5.0 TB/s   60          81                19
 //   Q4_0             38 (53)  3.4 TB/s   58          82 (590)          18
