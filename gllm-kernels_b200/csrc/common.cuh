@@ -119,6 +119,10 @@ struct Ctx {
     int64_t gemm_pdl = 1;        // weight-only GEMM launched programmatically behind its activation staging kernel
     int64_t raw_gemv_mma = 1;    // Q4_0 / Q5_0 rows of whole 256-element groups: 0 = the dp2a kernel (the other row-major formats have one kernel)
     int64_t gemm_row_tiles = 0;  // weight-only GEMM: row tiles per CTA (0 = estimated, 1, 2)
+    // The context has launched a wait for another rank.  What is queued behind one must not hold the SMs for as long as it lasts
+    // (kernels of other streams, perhaps those the other rank is waiting for, need them): staging kernels in front of the
+    // shared-memory-filling products are then launched plainly
+    bool peer_waits = false;
     int64_t peer_wait_spins = (int64_t)1 << 22;  // probes of another rank's flag before a wait gives up (status 31 / 32)
 };
 
@@ -153,9 +157,10 @@ struct DeviceGuard {
     } while (0)
 
 // Programmatic launch: the kernel starts as soon as every block of the kernel in front has issued
-// griddepcontrol.launch_dependents (or ended), and orders what it reads of it with griddepcontrol.wait.
+// griddepcontrol.launch_dependents (or ended), and orders what it reads of it with griddepcontrol.wait.  programmatic = false: a
+// plain launch, which starts when everything in front has ended.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_after(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+inline cudaError_t launch_after(void (*kern)(KArgs...), bool programmatic, dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)threads);
@@ -165,7 +170,7 @@ inline cudaError_t launch_after(void (*kern)(KArgs...), dim3 grid, int threads, 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = programmatic ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 

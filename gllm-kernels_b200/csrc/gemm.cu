@@ -636,11 +636,16 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
     tc::fence_after_sync();
     const uint32_t tmem_d = tmem_base_s;
     WQP_DECL;
+    // From here on every role executes griddepcontrol.wait before its first bounded wait that needs staged activations to end.  The
+    // grids in front may still be running, and one of them may be waiting (about a second, 2^22 probes with sleeps) for another
+    // rank; the probes below do not sleep and 2^22 of them are over in a tenth of that, so their bound must not start earlier.
+    // What runs ahead needs the first raw super-chunks only: their copies above and the conversion of each group's first A tile.
 
     if (warp == 0) {
         // ---------------- raw weight super-chunks, the rest ----------------
         // (row-major formats: the whole warp copies; the others: one thread's bulk copies)
         if (wq_row_major(FMT) || lane == 0) {
+            if (raw_pre < nraw) asm volatile("griddepcontrol.wait;\n" ::: "memory");
             int slot = raw_pre == p.r ? 0 : raw_pre, round = raw_pre == p.r ? 1 : 0;
             for (int q = raw_pre; q < nraw; q++) {
                 WQP_T0();
@@ -689,6 +694,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
         const int i = __shfl_sync(0xffffffffu, warp, 0) - 2;
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_d, 0);
         if (i < mt) {
+            asm volatile("griddepcontrol.wait;\n" ::: "memory");
             const uint32_t idesc = tc::idesc_f16(WQ_BM, ntile, 0, 0);  // fp16 x fp16 -> f32
             bool ok = true;
             int sb = 0, bround = 0;
@@ -758,6 +764,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
             }
             WQP_ACC(0);
             if (wg == 0) {
+                if (it == 1) asm volatile("griddepcontrol.wait;\n" ::: "memory");
                 bool ready = (it == 0 || tc::mbar_spin(emptyA + 8 * grp, (uint32_t)((it - 1) & 1), abort_flag));
                 WQP_ACC(1);
                 ready = ready && (a + 4 >= na || !last || tc::mbar_spin(rawfull + 8 * rslot, (uint32_t)(rround & 1), abort_flag));
@@ -784,6 +791,7 @@ __global__ void __launch_bounds__(WQ_THREADS, 1) gemm_wq_kernel(const __grid_con
             abort_s = 1;
             atomicExch(p.status, 13);
         }
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");
         ok = ok && !abort_s && tc::mbar_wait(accum, 0u, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
@@ -1010,7 +1018,7 @@ static int32_t gemm_groups_chunk(Ctx *c, const Weight *const *ws, int ng, const 
     int32_t rc = ensure_act(c, (size_t)nimg * nks * WQ_TILE);
     if (rc) return rc;
     p.xt = static_cast<const uint8_t *>(c->act);
-    GK_CUDA(c, launch_after(stage_act_kernel, dim3((unsigned)nks, (unsigned)nimg), 256, 0, s, a, a_bf16, lda, (int64_t)w->k,
+    GK_CUDA(c, launch_after(stage_act_kernel, !c->peer_waits, dim3((unsigned)nks, (unsigned)nimg), 256, 0, s, a, a_bf16, lda, (int64_t)w->k,
                             static_cast<uint8_t *>(c->act), imgs, a_up, wq_quads(fmt) ? 1 : 0));
     dim3 grid((unsigned)ntiles, (unsigned)((row_tiles + mt - 1) / mt));
     // Tail split: the last, partly filled wave of tiles — the only one, when there are fewer tiles than SMs — is cut along

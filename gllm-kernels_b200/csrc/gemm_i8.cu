@@ -211,6 +211,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) gemm_i8_kernel(const __grid_con
         // ---------------- MMA issue: weights signed (operand A), activations unsigned (operand B) ----------------
         // (the whole warp walks the k-steps, one elected lane issues: addresses and descriptors are uniform values)
         const uint32_t idesc = tc::idesc_i8(I8_BM, ntok, 1, 0), tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the bound of the waits starts when the images exist
         for (int ks = 0; ks < p.nks; ks++) {
             const int s = ks % I8_STAGES;
             if (!tc::mbar_spin_warp(full + 8 * s, (uint32_t)((ks / I8_STAGES) & 1), abort_flag)) {
@@ -240,6 +241,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) gemm_i8_kernel(const __grid_con
     if (warp >= 2) {
         // ---------------- epilogue: warp w reads TMEM lane quadrant w % 4 = weight rows ----------------
         const int quad = warp & 3;
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");  // as the MMA warp; and this thread reads the activation scale
         bool ok = !abort_s && tc::mbar_wait(accum, 0u, abort_flag);
         if (!ok && !abort_s) {
             abort_s = 1;
@@ -247,7 +249,6 @@ __global__ void __launch_bounds__(I8_THREADS, 1) gemm_i8_kernel(const __grid_con
         }
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
-            asm volatile("griddepcontrol.wait;\n" ::: "memory");  // this thread reads the activation scale
             tc::fence_after_sync();
             // all MMAs have completed, so the stages are free: each warp stages its blocks in 4 KB of stage 0
             uint8_t *stage = smem_raw + (smem_s - tc::smem_u32(smem_raw)) + (warp - 2) * 4096;
@@ -351,6 +352,7 @@ gemm_i8_pair_kernel(const __grid_constant__ I8Params p, const int tok_tiles, con
         // ---------------- partner CTA: tell the leader when this CTA's stage has landed ----------------
         uint32_t g = 0;
         bool ok = true;
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the bound of the waits starts when the images exist
         for (int t = pair; t < ntiles && ok && !*abort_flag; t += npairs)
             for (int ks = 0; ks < p.nks; ks++, g++) {
                 const uint32_t s = g % I8P_STAGES;
@@ -368,6 +370,7 @@ gemm_i8_pair_kernel(const __grid_constant__ I8Params p, const int tok_tiles, con
         // (the whole warp walks the k-steps, one elected lane issues: addresses and descriptors are uniform values)
         const uint32_t idesc = tc::idesc_i8(256, I8_BN, 1, 0);  // weights signed (operand A), activations unsigned (operand B)
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the bound of the waits starts when the images exist
         uint32_t g = 0, it = 0;
         bool ok = true;
         for (int t = pair; t < ntiles && ok; t += npairs, it++) {
@@ -583,8 +586,8 @@ static int32_t act_quant(Ctx *c, const float *x, int64_t rows, int64_t k, int64_
         const int64_t nr = rows - r0 < step ? rows - r0 : step;
         const dim3 grid((unsigned)((k + 127) / 128), (unsigned)((nr + 8 * AQ_ROWS - 1) / (8 * AQ_ROWS)));
         uint8_t *dst = img ? q + (size_t)(r0 >> 7) * ((size_t)(k + 127) / 128) * I8_TILE : q + r0 * ldq;
-        GK_CUDA(c, img ? launch_after(act_quant_i8_kernel<true>, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, amax, scale_dev)
-                       : launch_after(act_quant_i8_kernel<false>, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, amax, scale_dev));
+        GK_CUDA(c, img ? launch_after(act_quant_i8_kernel<true>, true, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, amax, scale_dev)
+                       : launch_after(act_quant_i8_kernel<false>, true, grid, 256, 0, s, x + r0 * ld, nr, k, ld, vec, dst, ldq, qvec, offset, amax, scale_dev));
     }
     return GLLMK_STATUS_OK;
 }
@@ -601,7 +604,7 @@ static int32_t i8_launch_mt(Ctx *c, const I8Params &p, dim3 grid, int ntok, cuda
         GK_CUDA(c, cudaFuncSetAttribute(gemm_i8_kernel<MT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)i8_smem<MT>()));
         attr_set[dev_slot] = true;
     }
-    GK_CUDA(c, launch_after(gemm_i8_kernel<MT, EPI>, grid, I8_THREADS, i8_smem<MT>(), s, p, ntok));
+    GK_CUDA(c, launch_after(gemm_i8_kernel<MT, EPI>, true, grid, I8_THREADS, i8_smem<MT>(), s, p, ntok));
     return GLLMK_STATUS_OK;
 }
 
@@ -656,7 +659,7 @@ static int32_t i8_product(Ctx *c, const Weight *w, I8Params p, int m, cudaStream
         }
         const int ntiles = pairs * mtiles;
         const int npairs = ntiles < pairs_resident[dev_slot] ? ntiles : pairs_resident[dev_slot];
-        GK_CUDA(c, launch_after(gemm_i8_pair_kernel<EPI>, dim3(2u * (unsigned)npairs), I8P_THREADS, I8P_SMEM, s, p, mtiles, i8_act_tiles(m)));
+        GK_CUDA(c, launch_after(gemm_i8_pair_kernel<EPI>, true, dim3(2u * (unsigned)npairs), I8P_THREADS, I8P_SMEM, s, p, mtiles, i8_act_tiles(m)));
         return GLLMK_STATUS_OK;
     }
     if (ntok > 128 && t2 < t1) return i8_launch_mt<2, EPI>(c, p, dim3((unsigned)pairs, (unsigned)mtiles), ntok, s);

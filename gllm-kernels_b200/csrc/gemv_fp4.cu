@@ -265,6 +265,9 @@ __global__ void __launch_bounds__(FD_THREADS, 1) gemv_fp4_tc_kernel(const __grid
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_base_s;
+    // Every role but the copies has nothing to do before the digit planes exist, and its bounded waits must not start earlier: the
+    // grids in front may still be waiting for another rank (about a second; the MMA warp's probes are over in a tenth of that).
+    if (warp != 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
     if (warp == 0) {
         if (lane == 0) {

@@ -359,7 +359,7 @@ int32_t quantize_launch(Ctx *c, int32_t qt, const float *x, int64_t rows, int64_
         const int vec = ((uintptr_t)x & 15) == 0;
         uint8_t *out = static_cast<uint8_t *>(blocks);
         if (given) quantize_nvfp4_kernel<<<grid, 256, 0, s>>>(x, vec, out, nullptr, *global_scale, units);
-        else GK_CUDA(c, launch_after(quantize_nvfp4_kernel, dim3(grid), 256, 0, s, x, vec, out, &amax_out(c)->global, 0.0f, units));
+        else GK_CUDA(c, launch_after(quantize_nvfp4_kernel, true, dim3(grid), 256, 0, s, x, vec, out, &amax_out(c)->global, 0.0f, units));
         GK_CUDA(c, cudaGetLastError());
         if (!given) {
             GK_CUDA(c, cudaEventSynchronize(c->host_word_ready));

@@ -180,6 +180,51 @@ def test_bounded_wait_runs_out_and_the_context_recovers(gk, K, oracle):
     w.free()
 
 
+@pytest.mark.parametrize("own_context", [True, False])
+def test_products_behind_a_rank_that_comes_late(gk, K, oracle, own_context):
+    """A barrier whose flag arrives 300 ms late (a 4-byte copy from page-locked memory stands in for the other rank), with every
+    product that is launched programmatically queued behind it: the products' own bounded waits (some tens of milliseconds of
+    back-to-back probes) must not run while the barrier still waits.  Status 0 and the results of an undisturbed run, bit for bit.
+    own_context: the barrier is launched by the products' context, which then launches its staging plainly, or by another one."""
+    import time
+    import torch
+    rng = np.random.default_rng(71)
+    prod = gk.GpuKernels(0)
+    barrier = (prod if own_context else K).peer_barrier
+    n, k = 640, 2048
+    runs = []
+    for fmt, m in (("q4k", 64), ("q4k", 300), ("mxfp4", 40), ("q6k", 48), ("nvfp4", 3), ("mxfp4", 1), ("q5k", 2), ("q8_0", 5)):
+        qt, _, blocks, scales, g = weight(gk, oracle, fmt, n, k, seed=72 + m)
+        w = prod.upload(qt, n, k, blocks, scales, g)
+        x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda()
+        runs.append((lambda w=w, x=x: prod.gemm(w, x)) if m > 16 else (lambda w=w, x=x: prod.gemv(w, x)))
+    w8 = prod.upload_int8(rng.integers(-128, 128, size=(n, k), dtype=np.int8), layout_kn=False)
+    xs = torch.from_numpy(rng.standard_normal((300, k)).astype(np.float32)).cuda()
+    runs.append(lambda: prod.w8a8_linear(w8, xs, 0.01))
+    before = [r().clone() for r in runs]  # scratch has its size from here on: nothing below waits for the device
+    mine = torch.zeros(64, dtype=torch.int32, device="cuda")
+    other = torch.zeros(64, dtype=torch.int32, device="cuda")
+    one = torch.ones(1, dtype=torch.int32).pin_memory()
+    late = torch.cuda.Stream()
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    for i, r in enumerate(runs):
+        seq = i + 1
+        one.fill_(seq)
+        torch.cuda.synchronize()
+        e0.record()
+        barrier(mine.data_ptr(), [other.data_ptr()], rank=0, seq=seq)
+        y = r()
+        e1.record()
+        time.sleep(0.3)
+        with torch.cuda.stream(late):
+            mine[1:2].copy_(one, non_blocking=True)
+        torch.cuda.synchronize()
+        assert e0.elapsed_time(e1) > 250.0  # the product did sit behind a waiting barrier
+        assert prod.status() == 0 and K.status() == 0
+        assert torch.equal(y, before[i])
+    prod.close()
+
+
 @pytest.mark.parametrize("fmt", ["q4k", "mxfp4"])
 def test_give_up_leaves_dirty_counters_and_status_read_restores_them(gk, K, oracle, fmt):
     """A decode kernel that gives up a wait leaves its row tiles' arrival counters non-zero.  The state is injected
