@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "device_pool.cuh"
 
 namespace gllmk {
 
@@ -61,85 +62,7 @@ int32_t ensure_host_word(Ctx *c) {
 }
 int32_t ensure_dev_io(Ctx *c, size_t bytes) { return grow(c, &c->dev_io, &c->dev_io_bytes, bytes, false); }
 
-// ---- device memory of weights ----
-// cudaMalloc and cudaFree each cost tens to hundreds of microseconds and cudaFree waits for the device, which is nothing for a
-// model's weights but most of the time of a call whose activations are quantized and uploaded like a weight
-// (gllmk_gemm_fp4: W[14336, 4096] x 2048 tokens 850 - 1360 us, 600 of them here).  Freed buffers of up to 64 MB therefore stay
-// with the library, at most 128 MB per device, until the last context of the device is freed or an allocation fails.  A buffer
-// that is taken again may still be read by kernels its last owner launched, on any stream: the taker waits for the device once
-// (an upload from device memory has to anyway).
-constexpr size_t POOL_MAX_BLOCK = (size_t)64 << 20, POOL_MAX_BYTES = (size_t)128 << 20;
-struct WeightPool {
-    struct Block { void *p; size_t bytes; };
-    std::mutex mu;
-    std::vector<Block> blocks;  // oldest first
-    size_t held = 0;
-    int contexts = 0;
-};
-static WeightPool &pool_of(int device) {
-    static WeightPool *pools = new WeightPool[64];  // never destroyed: weights may be freed while the process ends
-    return pools[device & 63];
-}
-// sizes are rounded up to an eighth of a power of two, so that token counts that differ a little share buffers
-static size_t pool_size(size_t bytes) {
-    if (bytes > POOL_MAX_BLOCK) return bytes;
-    size_t step = 4096;
-    while (step * 8 < bytes) step *= 2;
-    return (bytes + step - 1) / step * step;
-}
-static void pool_trim(int device) {
-    WeightPool &p = pool_of(device);
-    std::lock_guard<std::mutex> l(p.mu);
-    for (const WeightPool::Block &b : p.blocks) cudaFree(b.p);
-    p.blocks.clear();
-    p.held = 0;
-}
-// A buffer of at least *bytes (set to its size).  *waited: the device has been waited for.
-static cudaError_t pool_take(int device, size_t *bytes, void **out, bool *waited) {
-    *bytes = pool_size(*bytes);
-    *out = nullptr;
-    WeightPool &p = pool_of(device);
-    {
-        std::lock_guard<std::mutex> l(p.mu);
-        for (size_t i = p.blocks.size(); i-- > 0;)
-            if (p.blocks[i].bytes == *bytes) {
-                *out = p.blocks[i].p;
-                p.blocks.erase(p.blocks.begin() + (ptrdiff_t)i);
-                p.held -= *bytes;
-                break;
-            }
-    }
-    if (*out) {
-        const cudaError_t e = cudaDeviceSynchronize();
-        if (e == cudaSuccess) *waited = true;
-        else cudaFree(*out), *out = nullptr;
-        return e;
-    }
-    cudaError_t e = cudaMalloc(out, *bytes);
-    if (e == cudaErrorMemoryAllocation) {
-        (void)cudaGetLastError();
-        pool_trim(device);
-        e = cudaMalloc(out, *bytes);
-    }
-    return e;
-}
-static void pool_put(int device, void *ptr, size_t bytes) {
-    if (!ptr) return;
-    WeightPool &p = pool_of(device);
-    std::lock_guard<std::mutex> l(p.mu);
-    if (bytes > POOL_MAX_BLOCK || p.contexts == 0) {
-        cudaFree(ptr);
-        return;
-    }
-    while (p.held + bytes > POOL_MAX_BYTES) {
-        cudaFree(p.blocks.front().p);
-        p.held -= p.blocks.front().bytes;
-        p.blocks.erase(p.blocks.begin());
-    }
-    p.blocks.push_back({ptr, bytes});
-    p.held += bytes;
-}
-
+// ---- device memory of weights (device_pool.cuh) ----
 // Device buffers of a weight whose plane sizes are set: one allocation, the auxiliary plane behind the main one.
 static int32_t weight_buffers(Ctx *c, Weight *w, bool *waited) {
     const size_t aux_off = (w->qs_bytes + 255) & ~(size_t)255;
@@ -314,7 +237,7 @@ int32_t gllmk_ctx_create(int32_t device, gllmk_ctx *out) {
         return GLLMK_STATUS_RUNTIME_ERROR;
     }
     {
-        WeightPool &pool = pool_of(device);
+        DevicePool &pool = pool_of(device);
         std::lock_guard<std::mutex> l(pool.mu);
         pool.contexts++;
     }
@@ -329,7 +252,7 @@ void gllmk_ctx_free(gllmk_ctx ctx) {
     cudaDeviceSynchronize();
     bool last;
     {
-        WeightPool &pool = pool_of(c->device);
+        DevicePool &pool = pool_of(c->device);
         std::lock_guard<std::mutex> l(pool.mu);
         last = --pool.contexts == 0;
     }

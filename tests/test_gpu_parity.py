@@ -581,3 +581,18 @@ def test_matmul_host_results_up_to_half_a_megabyte_are_stored_directly(gk, K, or
     assert np.array_equal(out, K.gemv(w, torch.from_numpy(x).cuda()).cpu().numpy())
     assert K.status() == 0
     w.free()
+
+
+@pytest.mark.parametrize("fmt,n,k", [("q4k", 14336, 4096), ("mxfp4", 14336, 4096), ("q8_0", 4096, 4096)])
+def test_a_weight_takes_no_more_device_memory_than_it_holds(gk, K, torch, fmt, n, k):
+    """A model's weights, uploaded one after the other from device memory and kept.  The driver hands out pages of 2 MB."""
+    qt = {"q4k": gk.QuantType.q4k(), "q8_0": gk.QuantType.q8_0(), "mxfp4": gk.QuantType.mxfp4(32)}[fmt]
+    got = K.quantize(qt, torch.zeros((n, k), device="cuda"))
+    blocks, scales = got if fmt == "mxfp4" else (got, None)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ws = [K.upload(qt, n, k, blocks, scales) for _ in range(4)]
+    took = free - torch.cuda.mem_get_info()[0]
+    assert took <= sum(w.info()["dev_bytes"] for w in ws) + 4 * (2 << 20)
+    for w in ws:
+        w.free()
