@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "tc05.cuh"
 
+#include <cfloat>
 #include <type_traits>
 
 namespace gllmk {
@@ -52,9 +53,11 @@ struct I8Params {
 // cancellation for negative u).  The quotient is Markstein's (q = v y, q += (v - q d) y, y an approximate 1 / d): no branch,
 // so the chains of a thread's 32 elements overlap; the compiler's IEEE division has one per element, and the fused
 // epilogue of gemm_i8_pair_kernel then took 134 us on W[11008, 4096] x 2048 (82 now; the product without it 72).
+// v and q infinite (v = inf, d = 1) or exp overflown (d = inf, y = 0): the residual is the NaN of inf - inf or 0 * inf.  fmax takes
+// the other operand then, and q is the answer (inf, or 0).
 __device__ __forceinline__ float sigmoid_times(float v, float z) {
     const float d = 1.0f + expf(-z), y = __fdividef(1.0f, d), q = v * y;
-    return d < 1e37f ? fmaf(fmaf(-q, d, v), y, q) : q;  // exp overflows: y = 0, and the residual would be 0 * inf
+    return d < 1e37f ? fmaf(fmaxf(fmaf(-q, d, v), -FLT_MAX), y, q) : q;
 }
 // dequantize_i32_to_f32 (src/macros/matmul_x86_int8.rs:414-456, scalar tail semantics): (c as f32) * scale_a * scale_b
 // (+ bias[j]), then the activation of src/macros/gemm_epilogue.rs:131-152

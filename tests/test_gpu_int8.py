@@ -124,6 +124,29 @@ def test_dequantize_epilogue(gk, K):
     assert np.allclose(gelu, 0.5 * v * (1.0 + np.tanh(inner)), rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("act", [2, 3, 4])
+def test_epilogue_activations_at_infinity(gk, K, act):
+    """SiLU and GELU of what an overflowing product or an infinite bias leaves: the IEEE quotient v / (1 + exp(-z)) as the
+    reference's epilogue has it, in the dequantize pass and in the fused layer.  +inf stays +inf, NaN stays NaN, -inf gives the
+    quotient's NaN, and the largest finite values go to themselves and to zero."""
+    import torch
+    inf, big = np.float32(np.inf), np.finfo(np.float32).max
+    v = np.array([inf, -inf, np.nan, big, -big, 88.0, 0.0, -0.0], np.float32)
+    ref = np.array([inf, np.nan, np.nan, big, 0.0, 88.0, 0.0, 0.0], np.float32)
+    n = v.size
+    bias = torch.from_numpy(v).cuda()
+    zero = torch.zeros((3, n), dtype=torch.int32, device="cuda")
+    w = K.upload_int8(np.zeros((n, 32), np.int8), layout_kn=False)
+    for y in (K.dequantize_i32(zero, 1.0, 1.0, bias=bias, activation=act), K.w8a8_linear(w, torch.ones((3, 32), device="cuda"), 1.0, bias=bias, activation=act)):
+        for row in y.cpu().numpy():
+            np.testing.assert_array_equal(row, ref)  # NaN equals NaN here, -0 equals 0
+    # a product that overflows: (c as f32) * scale_a * scale_b
+    c = torch.tensor([[1 << 30, -(1 << 30)]], dtype=torch.int32, device="cuda")
+    got = K.dequantize_i32(c, 1e20, 1e20, activation=act).cpu().numpy()[0]
+    assert got[0] == inf and np.isnan(got[1])
+    w.free()
+
+
 def test_int8_argument_checks(gk, K, oracle):
     import torch
     with pytest.raises(gk.GllmkError) as e:
