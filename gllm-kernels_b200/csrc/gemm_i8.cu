@@ -53,11 +53,16 @@ struct I8Params {
 // cancellation for negative u).  The quotient is Markstein's (q = v y, q += (v - q d) y, y an approximate 1 / d): no branch,
 // so the chains of a thread's 32 elements overlap; the compiler's IEEE division has one per element, and the fused
 // epilogue of gemm_i8_pair_kernel then took 134 us on W[11008, 4096] x 2048 (82 now; the product without it 72).
+// y comes from d / 8, because 1 / d itself would be 0 from d = 2^126 on (SiLU(-88) = -0 instead of -5e-37).
 // v and q infinite (v = inf, d = 1) or exp overflown (d = inf, y = 0): the residual is the NaN of inf - inf or 0 * inf.  fmax takes
 // the other operand then, and q is the answer (inf, or 0).
 __device__ __forceinline__ float sigmoid_times(float v, float z) {
-    const float d = 1.0f + expf(-z), y = __fdividef(1.0f, d), q = v * y;
-    return d < 1e37f ? fmaf(fmaxf(fmaf(-q, d, v), -FLT_MAX), y, q) : q;
+    const float d = 1.0f + expf(-z);
+    float y;  // 1 / 8 <= d / 8 <= 2^125: neither side of the reciprocal is subnormal
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d * 0.125f));
+    y *= 0.125f;
+    const float q = v * y;
+    return fmaf(fmaxf(fmaf(-q, d, v), -FLT_MAX), y, q);
 }
 // dequantize_i32_to_f32 (src/macros/matmul_x86_int8.rs:414-456, scalar tail semantics): (c as f32) * scale_a * scale_b
 // (+ bias[j]), then the activation of src/macros/gemm_epilogue.rs:131-152

@@ -147,6 +147,25 @@ def test_epilogue_activations_at_infinity(gk, K, act):
     w.free()
 
 
+@pytest.mark.parametrize("act", [2, 3])
+def test_epilogue_activations_where_the_exponential_nears_overflow(gk, K, act):
+    """Arguments whose exp(-z) lies between 1e26 and FLT_MAX (z = v for SiLU, twice the inner polynomial for GELU): the quotient
+    stays a normal number and keeps its relative error (expf 2 ulp, its argument's rounding amplified by |z| < 89:
+    89 * 2^-24 + 2^-22 < 5.6e-6 for SiLU; GELU's argument is itself rounded four times, 4 * 89 * 2^-24 more)."""
+    import torch
+    if act == 2:
+        v = np.linspace(-88.7, -60.0, 4001).astype(np.float32)
+        z = v.astype(np.float64)
+    else:
+        v = np.linspace(-10.05, -9.0, 4001).astype(np.float32)
+        z = 2 * np.float64(np.float32(0.7978845608)) * (v.astype(np.float64) + np.float64(np.float32(0.044715)) * v.astype(np.float64) ** 3)
+    assert z.min() > -88.72
+    ref = v / (1 + np.exp(-z))
+    y = K.dequantize_i32(torch.zeros((1, v.size), dtype=torch.int32, device="cuda"), 1.0, 1.0, bias=torch.from_numpy(v).cuda(), activation=act)
+    err = np.abs(y.cpu().numpy()[0] - ref) / np.abs(ref)
+    assert err.max() <= (5.6e-6 if act == 2 else 5.6e-6 + 4 * 89 * 2.0 ** -24)
+
+
 def test_int8_argument_checks(gk, K, oracle):
     import torch
     with pytest.raises(gk.GllmkError) as e:
