@@ -7,7 +7,9 @@
 //   * activations are three s8 digits per value and 256-element block, x = amax / 8355711 * (65536 d1 + 256 d2 + d3): 24 bits,
 //     rounding error 6e-8 of the block's maximum, and the three digits of a token are three COLUMNS of the product, each an
 //     activation vector of its own whose scale carries the digit's weight.  (s16 per 32 elements, the previous scheme, needs a
-//     conversion and a float scale per 32 weights, row and token.)
+//     conversion and a float scale per 32 weights, row and token.)  A block with a 32-element run whose maximum lies more than 255
+//     times below the block's — there s16 per run would be the finer form — carries what the three digits leave as a second
+//     slice of three more, and is walked twice: the error is nowhere larger than 16 bits per run gave.
 //   * Q5_K's 6-bit and Q6_K's 8-bit sub-scales multiply the s32 sums (one IMAD each), Q8_K chains the accumulator over the whole
 //     block, and only Q4_0 / Q5_0, whose scale is an f16 per 32 weights, go through f32 per MMA (the accumulator starts at
 //     1.5 * 2^23 so that its bits ARE a float: no conversion instruction).
@@ -19,11 +21,12 @@
 // in brackets the kernels before: dp2a on CUDA cores, and for Q6_K of two tokens and more an MMA kernel of 16 rows per CTA whose
 // warps staged the activations each for themselves:
 //   W[8192, 28672]   1 token            8 tokens     16 tokens         W[11008, 4096], 5 tokens
-//   Q6_K             49 (62)  3.9 TB/s   72 (100)    117 (135)         19
-//   Q5_K             44 (73)  3.6 TB/s   61          87 (590)          18 (61)
-//   Q8_K             53 (69)  5.0 TB/s   60          81                19
-//   Q4_0             38 (53)  3.4 TB/s   58          82 (590)          18
-//   Q5_0             51 (67)  3.2 TB/s   70          95 (590)          21
+//   Q6_K             50 (62)  3.9 TB/s   74 (100)    120 (135)         20
+//   Q5_K             45 (73)  3.6 TB/s   63          89 (590)          19 (61)
+//   Q8_K             54 (69)  4.9 TB/s   63          87                19
+//   Q4_0             39 (53)  3.3 TB/s   59          83 (590)          18
+//   Q5_0             54 (67)  3.0 TB/s   72          98 (590)          21
+// With a wide block in every CTA 1.7 times that (geometric mean); the flags and scales of the second slices cost the others 3 %.
 #include "common.cuh"
 
 namespace gllmk {
@@ -37,18 +40,54 @@ constexpr int RM_PASS = 16;    // tokens per pass
 __host__ __device__ constexpr int rm_groups(int m) { return (3 * m + 7) / 8; }  // MMA column groups
 // slice of one block: [3m][288] digits, [3m][16] digit sums of the eight 32-element runs (S = 64 hi + lo: 8 hi, 8 lo), [8 groups] f32
 __host__ __device__ constexpr uint32_t rm_slice_bytes(int m) { return (uint32_t)(3 * m) * (RM_PITCH + 16) + 32u * (uint32_t)rm_groups(m); }
+// image: a slice per block, then as many for the rests of wide blocks.  Token t's block is wide: the word behind its first column's digits
+__host__ __device__ constexpr size_t rm_image_bytes(int m, int64_t nb) { return 2 * (size_t)nb * rm_slice_bytes(m); }
+__host__ __device__ constexpr uint32_t rm_flag_at(int tok) { return (uint32_t)(3 * tok) * RM_PITCH + 256u; }
+constexpr float RM_WIDE = 255.0f;             // 8355711 / 32767: block maximum over a run's, from which on s16 per run is the finer form
+constexpr float RM_REST = 2.0f * 8355711.0f;  // the rest is at most half a step: digits of rest * RM_REST
 
 struct RmStage {
     const float *x;
     int64_t xst, xsk, k;
     int m, sums;
-    uint8_t *img;
+    uint8_t *img, *rest;
 };
+
+// q (24 bits, |q| <= 8355711) -> digit i of the three words, added to the digit sums
+__device__ __forceinline__ void rm_digits(int q, int i, uint32_t (&w)[3], int (&s)[3]) {
+    const int d3 = ((q + 128) & 255) - 128, q2 = (q - d3) >> 8;
+    const int d2 = ((q2 + 128) & 255) - 128, d1 = (q2 - d2) >> 8;
+    w[0] |= (uint32_t)(d1 & 255) << (8 * i);
+    w[1] |= (uint32_t)(d2 & 255) << (8 * i);
+    w[2] |= (uint32_t)(d3 & 255) << (8 * i);
+    s[0] += d1;
+    s[1] += d2;
+    s[2] += d3;
+}
+// The words of elements kk .. kk + 3 of a block, and (sums) the digit sums of the run's eight lanes
+__device__ __forceinline__ void rm_store(uint8_t *slice, int m, int tok, int kk, const uint32_t (&w)[3], int (&s)[3], int sums) {
+    const int ncol = 3 * m, run = kk >> 5, j = (kk >> 2) & 7;
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+        *reinterpret_cast<uint32_t *>(slice + (3 * tok + d) * RM_PITCH + 32 * run + 8 * (j & 3) + 4 * (j >> 2)) = w[d];
+    if (sums) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) s[d] += __shfl_xor_sync(0xffffffffu, s[d], o);
+            if (j == 0) {
+                uint8_t *sp = slice + ncol * RM_PITCH + (3 * tok + d) * 16;
+                sp[run] = (uint8_t)(int8_t)(s[d] >> 6);
+                sp[8 + run] = (uint8_t)(s[d] & 63);
+            }
+        }
+    }
+}
 
 // Thread = four elements; a CTA's 64 threads = one 256-element block.  In a run, elements 4t .. 4t + 3 and 16 + 4t .. + 3 are lane t's two
 // operand-B words (byte 8t of the run).
 __global__ void __launch_bounds__(64) raw_mma_stage_kernel(const RmStage p) {
-    __shared__ float wmax[2];
+    __shared__ float wmax[2], wmin[2];
     __shared__ int wbad[2];
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -69,55 +108,59 @@ __global__ void __launch_bounds__(64) raw_mma_stage_kernel(const RmStage p) {
     const float inf = __int_as_float(0x7F800000);
     int bad = !(fabsf(v[0]) < inf) || !(fabsf(v[1]) < inf) || !(fabsf(v[2]) < inf) || !(fabsf(v[3]) < inf);
 #pragma unroll
-    for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    for (int o = 1; o < 8; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    float low = amax > 0.0f ? amax : inf;  // smallest maximum of a run that is not all zero
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        low = fminf(low, __shfl_xor_sync(0xffffffffu, low, o));
+    }
     bad = __any_sync(0xffffffffu, bad);
-    if (lane == 0) { wmax[warp] = amax; wbad[warp] = bad; }
+    if (lane == 0) { wmax[warp] = amax; wmin[warp] = low; wbad[warp] = bad; }
     __syncthreads();
     if (k0 >= p.k) return;
-    amax = fmaxf(wmax[warp & ~1], wmax[warp | 1]);
-    bad = wbad[warp & ~1] | wbad[warp | 1];
+    amax = fmaxf(wmax[0], wmax[1]);
+    bad = wbad[0] | wbad[1];
+    const bool wide = !bad && amax > RM_WIDE * fminf(wmin[0], wmin[1]);
     // tiny blocks are pre-scaled by 2^64 so that 8355711 / amax stays finite
     const float pre = amax < 1e-20f ? 18446744073709551616.0f : 1.0f;
     const float inv = (amax > 0.0f && !bad) ? 8355711.0f / (amax * pre) : 0.0f;
     uint32_t w[3] = {0, 0, 0};
     int s[3] = {0, 0, 0};
+    float rest[4];  // what the digits leave, in steps: exact, |rest| <= 1/2
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int q = bad ? 0 : (int)fminf(fmaxf(rintf((v[i] * pre) * inv), -8355711.0f), 8355711.0f);
-        const int d3 = ((q + 128) & 255) - 128, q2 = (q - d3) >> 8;
-        const int d2 = ((q2 + 128) & 255) - 128, d1 = (q2 - d2) >> 8;
-        w[0] |= (uint32_t)(d1 & 255) << (8 * i);
-        w[1] |= (uint32_t)(d2 & 255) << (8 * i);
-        w[2] |= (uint32_t)(d3 & 255) << (8 * i);
-        s[0] += d1;
-        s[1] += d2;
-        s[2] += d3;
+        const float f = (v[i] * pre) * inv, r = fminf(fmaxf(rintf(f), -8355711.0f), 8355711.0f);
+        rest[i] = f - r;
+        rm_digits(bad ? 0 : (int)r, i, w, s);
     }
-    const int ncol = 3 * p.m, kk = (int)(k0 & 255), run = kk >> 5, j = (kk >> 2) & 7;
-    uint8_t *slice = p.img + (k0 >> 8) * (int64_t)rm_slice_bytes(p.m);
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-        *reinterpret_cast<uint32_t *>(slice + (3 * tok + d) * RM_PITCH + 32 * run + 8 * (j & 3) + 4 * (j >> 2)) = w[d];
-    if (p.sums) {
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-#pragma unroll
-            for (int o = 1; o < 8; o <<= 1) s[d] += __shfl_xor_sync(0xffffffffu, s[d], o);
-            if (j == 0) {
-                uint8_t *sp = slice + ncol * RM_PITCH + (3 * tok + d) * 16;
-                sp[run] = (uint8_t)(int8_t)(s[d] >> 6);
-                sp[8 + run] = (uint8_t)(s[d] & 63);
-            }
-        }
-    }
-    float *scales = reinterpret_cast<float *>(slice + ncol * (RM_PITCH + 16));
+    const int ncol = 3 * p.m, kk = (int)(k0 & 255);
+    const int64_t at = (k0 >> 8) * (int64_t)rm_slice_bytes(p.m);
+    uint8_t *slice = p.img + at, *slice2 = p.rest + at;
+    rm_store(slice, p.m, tok, kk, w, s, p.sums);
+    const uint32_t scales = (uint32_t)ncol * (RM_PITCH + 16);
     if (kk < 12) {  // three threads: one digit's column each
         const float unit = kk == 0 ? 65536.0f / 8355711.0f : (kk == 4 ? 256.0f / 8355711.0f : 1.0f / 8355711.0f);
-        scales[3 * tok + (kk >> 2)] = bad ? __int_as_float(0x7FC00000) : amax * unit;
+        const uint32_t at_col = scales + 4 * (3 * tok + (kk >> 2));
+        // an all-zero block: digits 0, times 1, so that an infinite weight scale still gives NaN
+        *reinterpret_cast<float *>(slice + at_col) = bad ? __int_as_float(0x7FC00000) : (amax > 0.0f ? amax * unit : 1.0f);
+        // 0: when another token's block is wide, this token's second slice is read too, and not written
+        *reinterpret_cast<float *>(slice2 + at_col) = wide ? amax * (unit * (1.0f / RM_REST)) : 0.0f;
     }
+    if (kk == 16) *reinterpret_cast<uint32_t *>(slice + rm_flag_at(tok)) = wide ? 1u : 0u;
     if (tok == 0 && kk >= 32 && kk < 64) {  // columns that only fill up the last group: at most seven
         const int col = ncol + ((kk - 32) >> 2);
-        if (col < 8 * rm_groups(p.m)) scales[col] = 0.0f;
+        if (col < 8 * rm_groups(p.m)) {
+            *reinterpret_cast<float *>(slice + scales + 4 * col) = 0.0f;
+            *reinterpret_cast<float *>(slice2 + scales + 4 * col) = 0.0f;
+        }
+    }
+    if (wide) {  // the CTA as a whole
+        w[0] = w[1] = w[2] = 0;
+        s[0] = s[1] = s[2] = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) rm_digits((int)fminf(fmaxf(rintf(rest[i] * RM_REST), -8355711.0f), 8355711.0f), i, w, s);
+        rm_store(slice2, p.m, tok, kk, w, s, p.sums);
     }
 }
 
@@ -192,15 +235,20 @@ __device__ __forceinline__ uint32_t col_addr(const RmCols &x, int ng) { return n
 template <int NG>
 __device__ __forceinline__ uint32_t sum_addr(const RmCols &x, int ng) { return ng == NG - 1 ? x.sum_last : x.sum_first + (uint32_t)(ng * 8 * 16); }
 
-// tot[ng][0, 1]: row g, columns 8 ng + 2t, + 1; [2, 3]: row g + 8
-template <int NG>
+// tot[ng][0, 1]: row g, columns 8 ng + 2t, + 1; [2, 3]: row g + 8.  REST (x may be a second slice): a column of scale 0 has no rest
+// and adds nothing, whatever the slice holds there and the weight's scale is (0 * inf).
+template <int NG, bool REST>
 __device__ __forceinline__ void add_scaled(const RmCols &x, int t, int ng, const float (&f)[4], float (&tot)[NG][4]) {
     const uint2 s = lds64(x.scales + 32 * ng + 8 * t);
     const float sa = __uint_as_float(s.x), sb = __uint_as_float(s.y);
-    tot[ng][0] = fmaf(sa, f[0], tot[ng][0]);
-    tot[ng][1] = fmaf(sb, f[1], tot[ng][1]);
-    tot[ng][2] = fmaf(sa, f[2], tot[ng][2]);
-    tot[ng][3] = fmaf(sb, f[3], tot[ng][3]);
+    if (!REST || sa != 0.0f) {
+        tot[ng][0] = fmaf(sa, f[0], tot[ng][0]);
+        tot[ng][2] = fmaf(sa, f[2], tot[ng][2]);
+    }
+    if (!REST || sb != 0.0f) {
+        tot[ng][1] = fmaf(sb, f[1], tot[ng][1]);
+        tot[ng][3] = fmaf(sb, f[3], tot[ng][3]);
+    }
 }
 
 // Per format: BYTES of a row per 256 elements, CH 16-byte copies per row and block, PITCH of a row in shared memory (the 16 bytes
@@ -213,7 +261,7 @@ template <>
 struct Rm<GLLMK_QUANT_Q5_K> {
     static constexpr int BYTES = 176, CH = 11, PITCH = 176;
     static constexpr bool ALIGNED = true;
-    template <int NG>
+    template <int NG, bool REST>
     static __device__ __forceinline__ void block(uint32_t r0, uint32_t r8, int t, const RmCols &x, float (&tot)[NG][4]) {
         static_assert(FD_Q5K.scale_offset == 0 && FD_Q5K.scale_min_offset == 2 && FD_Q5K.sub_scales_offset == 4 && FD_Q5K.data_high_offset == 16,
                       "Q5_K header is the block's first 16 bytes");
@@ -266,7 +314,7 @@ struct Rm<GLLMK_QUANT_Q5_K> {
                                 fmaf(d0, (float)acc[ng][1], -(mn0 * (float)(64 * hi[1] + lo[1]))),
                                 fmaf(d8, (float)acc[ng][2], -(mn8 * (float)(64 * hi[2] + lo[2]))),
                                 fmaf(d8, (float)acc[ng][3], -(mn8 * (float)(64 * hi[3] + lo[3])))};
-            add_scaled<NG>(x, t, ng, f, tot);
+            add_scaled<NG, REST>(x, t, ng, f, tot);
         }
     }
 };
@@ -279,7 +327,7 @@ struct Rm<GLLMK_QUANT_Q6_K> {
     static __device__ __forceinline__ uint32_t word(uint32_t lo, uint32_t hi) {
         return ((lo & 0x3C3C3C3Cu) | 0x80808080u) ^ (hi & 0xC0C0C0C0u);
     }
-    template <int NG>
+    template <int NG, bool REST>
     static __device__ __forceinline__ void block(uint32_t r0, uint32_t r8, int t, const RmCols &x, float (&tot)[NG][4]) {
         const uint4 S0 = lds128(r0 + FD_Q6K.sub_scales_offset), S8 = lds128(r8 + FD_Q6K.sub_scales_offset);
         const uint32_t s0w[4] = {S0.x, S0.y, S0.z, S0.w}, s8w[4] = {S8.x, S8.y, S8.z, S8.w};
@@ -330,7 +378,7 @@ struct Rm<GLLMK_QUANT_Q6_K> {
 #pragma unroll
         for (int ng = 0; ng < NG; ng++) {
             const float f[4] = {d0 * (float)acc[ng][0], d0 * (float)acc[ng][1], d8 * (float)acc[ng][2], d8 * (float)acc[ng][3]};
-            add_scaled<NG>(x, t, ng, f, tot);
+            add_scaled<NG, REST>(x, t, ng, f, tot);
         }
     }
 };
@@ -340,7 +388,7 @@ struct Rm<GLLMK_QUANT_Q8_K> {
     // 292-byte blocks: a copy starts at the 16-byte boundary below the block
     static constexpr int BYTES = 292, CH = 19, PITCH = 304;
     static constexpr bool ALIGNED = false;
-    template <int NG>
+    template <int NG, bool REST>
     static __device__ __forceinline__ void block(uint32_t r0, uint32_t r8, int t, const RmCols &x, float (&tot)[NG][4]) {
         const uint32_t ra = r0 + FD_Q8K.data_offset + 4 * t, rb = r8 + FD_Q8K.data_offset + 4 * t;
         int acc[NG][4];
@@ -356,7 +404,7 @@ struct Rm<GLLMK_QUANT_Q8_K> {
 #pragma unroll
         for (int ng = 0; ng < NG; ng++) {
             const float f[4] = {d0 * (float)acc[ng][0], d0 * (float)acc[ng][1], d8 * (float)acc[ng][2], d8 * (float)acc[ng][3]};
-            add_scaled<NG>(x, t, ng, f, tot);
+            add_scaled<NG, REST>(x, t, ng, f, tot);
         }
     }
 };
@@ -372,7 +420,7 @@ struct RmClassic {
     static constexpr int BB = Q5 ? FD_Q5_0.block_bytes : FD_Q4_0.block_bytes, DATA = Q5 ? FD_Q5_0.data_offset : FD_Q4_0.data_offset;
     static constexpr int BYTES = 8 * BB, CH = BYTES / 16, PITCH = BYTES;
     static constexpr bool ALIGNED = true;
-    template <int NG>
+    template <int NG, bool REST>
     static __device__ __forceinline__ void block(uint32_t r0, uint32_t r8, int t, const RmCols &x, float (&tot)[NG][4]) {
         float cs[NG][4];
 #pragma unroll
@@ -410,7 +458,7 @@ struct RmClassic {
             }
         }
 #pragma unroll
-        for (int ng = 0; ng < NG; ng++) add_scaled<NG>(x, t, ng, cs[ng], tot);
+        for (int ng = 0; ng < NG; ng++) add_scaled<NG, REST>(x, t, ng, cs[ng], tot);
     }
 };
 template <>
@@ -420,7 +468,7 @@ struct Rm<GLLMK_QUANT_Q5_0> : RmClassic<GLLMK_QUANT_Q5_0> {};
 
 struct RmParams {
     const uint8_t *w;
-    const uint8_t *img;
+    const uint8_t *img, *rest;
     float *y;
     const float *row_scales;
     int64_t n_row_scales;
@@ -520,7 +568,12 @@ __host__ __device__ constexpr size_t rm_smem_bytes(int m, int stages) {
 __host__ __device__ constexpr int rm_min_ctas(int ng) { return ng <= 2 ? 3 : 2; }
 
 template <int QT, int NG>
-__global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_kernel(const __grid_constant__ RmParams p) {
+__device__ __noinline__ void rm_wide(const RmParams &p, int i0);
+
+// The CTA's units from number i0 on.  WIDE: i0 is a wide block whose first walk is done, with the sums so far in `red`; wide blocks are
+// walked twice.
+template <int QT, int NG, bool WIDE>
+__device__ __forceinline__ void rm_body(const RmParams &p, const int i0) {
     using F = Rm<QT>;
     constexpr int CH = F::CH;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -529,9 +582,8 @@ __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_k
     const uint32_t slice = rm_slice_bytes(p.m), stage = RM_ROWS * F::PITCH + slice;
     const uint32_t base = sm_addr(smem), zero = base + S * stage;
     float *red = reinterpret_cast<float *>(smem + (size_t)S * stage + 256) + warp * 16 * (8 * NG + 1);
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    const int64_t u0 = (int64_t)blockIdx.x * p.per_cta + min((int)blockIdx.x, p.rem);
-    const int n = p.per_cta + ((int)blockIdx.x < p.rem ? 1 : 0);
+    const int64_t u0 = (int64_t)blockIdx.x * p.per_cta + min((int)blockIdx.x, p.rem) + i0;
+    const int n = p.per_cta + ((int)blockIdx.x < p.rem ? 1 : 0) - i0;
 
     // ---- copies: the producer's position runs S - 1 steps ahead of the consumer's ----
     // Half a warp per row piece (a whole one for Q8_K's nineteen 16-byte chunks): lane = chunk, so a copy is one instruction and one
@@ -602,9 +654,13 @@ __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_k
     }
 
     const bool last_on = (NG - 1) * 8 + g < ncol;
+    // row g (+ 8), column 8 ng + 2t (+ 1) of the warp's sums
+    const auto red_at = [&](int ng, int j) -> float & { return red[(g + 8 * (j >> 1)) * (8 * NG + 1) + 8 * ng + 2 * t + (j & 1)]; };
     float tot[NG][4];
 #pragma unroll
-    for (int ng = 0; ng < NG; ng++) tot[ng][0] = tot[ng][1] = tot[ng][2] = tot[ng][3] = 0.0f;
+    for (int ng = 0; ng < NG; ng++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) tot[ng][j] = WIDE ? red_at(ng, j) : 0.0f;
     int64_t tg = u0 / nb;
     int b = (int)(u0 - tg * nb), st = 0;
     for (int i = 0; i < n; i++) {
@@ -621,22 +677,49 @@ __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_k
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         const int64_t row0 = tg * RM_ROWS + 16 * warp;
-        if (row0 < p.n) {
-            uint32_t r0 = base + st * stage + (16 * warp + g) * F::PITCH, r8 = r0 + 8 * F::PITCH;
-            if (!F::ALIGNED) {
-                // where the block starts in its first 16 bytes
-                const uint32_t ra = (uint32_t)reinterpret_cast<uintptr_t>(p.w) + (uint32_t)b * F::BYTES + (uint32_t)(row0 + g) * p.pitch;
-                r0 += ra & 15u;
-                r8 += (ra + 8 * p.pitch) & 15u;
+        const uint32_t xs = base + st * stage + RM_ROWS * F::PITCH;
+        const uint32_t flag = lds32(lane < p.m ? xs + rm_flag_at(lane) : zero);
+#pragma unroll 1
+        for (int pass = WIDE && i == 0 ? 1 : 0;; pass++) {
+            if (WIDE && pass > 0) {
+                // the rests take the slice's place in the stage
+                __syncthreads();
+                const uint8_t *src = p.rest + (size_t)b * slice;
+                for (uint32_t o = threadIdx.x * 16; o < slice; o += RM_WARPS * 32 * 16) {
+                    const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(src + o));
+                    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(xs + o), "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w) : "memory");
+                }
+                __syncthreads();
             }
-            const uint32_t xs = base + st * stage + RM_ROWS * F::PITCH;
-            RmCols x;
-            x.first = xs + g * RM_PITCH + 8 * t;
-            x.last = last_on ? x.first + (NG - 1) * 8 * RM_PITCH : zero;
-            x.sum_first = xs + ncol * RM_PITCH + g * 16;
-            x.sum_last = last_on ? x.sum_first + (NG - 1) * 8 * 16 : zero;
-            x.scales = xs + ncol * (RM_PITCH + 16);
-            F::template block<NG>(r0, r8, t, x, tot);
+            if (row0 < p.n) {
+                uint32_t r0 = base + st * stage + (16 * warp + g) * F::PITCH, r8 = r0 + 8 * F::PITCH;
+                if (!F::ALIGNED) {
+                    // where the block starts in its first 16 bytes
+                    const uint32_t ra = (uint32_t)reinterpret_cast<uintptr_t>(p.w) + (uint32_t)b * F::BYTES + (uint32_t)(row0 + g) * p.pitch;
+                    r0 += ra & 15u;
+                    r8 += (ra + 8 * p.pitch) & 15u;
+                }
+                RmCols x;
+                x.first = xs + g * RM_PITCH + 8 * t;
+                x.last = last_on ? x.first + (NG - 1) * 8 * RM_PITCH : zero;
+                x.sum_first = xs + ncol * RM_PITCH + g * 16;
+                x.sum_last = last_on ? x.sum_first + (NG - 1) * 8 * 16 : zero;
+                x.scales = xs + ncol * (RM_PITCH + 16);
+                F::template block<NG, WIDE>(r0, r8, t, x, tot);
+            }
+            if (!WIDE || pass > 0 || !__any_sync(0xffffffffu, flag != 0)) break;
+        }
+        if (!WIDE && __any_sync(0xffffffffu, flag != 0)) {
+            // A wide block (all warps see the same): the rest of the way out of line, for the plain loop's registers (second walk inside
+            // it: Q8_K W[8192, 28672] x 16 tokens 90 us, now 87; 83 without the second slice).
+#pragma unroll
+            for (int ng = 0; ng < NG; ng++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) red_at(ng, j) = tot[ng][j];
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            rm_wide<QT, NG>(p, i);
+            return;
         }
         st = st + 1 == S ? 0 : st + 1;
         if (++b == nb || i + 1 == n) {
@@ -647,7 +730,7 @@ __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_k
                 for (int ng = 0; ng < NG; ng++)
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        red[(g + 8 * (j >> 1)) * (8 * NG + 1) + 8 * ng + 2 * t + (j & 1)] = tot[ng][j];
+                        red_at(ng, j) = tot[ng][j];
                         tot[ng][j] = 0.0f;
                     }
                 __syncwarp();
@@ -658,6 +741,14 @@ __global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_k
             tg++;
         }
     }
+}
+template <int QT, int NG>
+__device__ __noinline__ void rm_wide(const RmParams &p, int i0) { rm_body<QT, NG, true>(p, i0); }
+
+template <int QT, int NG>
+__global__ void __launch_bounds__(RM_WARPS * 32, rm_min_ctas(NG)) raw_mma_gemv_kernel(const __grid_constant__ RmParams p) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    rm_body<QT, NG, false>(p, 0);
 }
 
 // Resident CTAs per SM and stages for (format, groups, tokens): as many CTAs as the registers allow with two stages, then as many
@@ -742,11 +833,10 @@ int32_t raw_mma_launch(Ctx *c, const Weight *w, const float *x, int64_t xst, int
                        const float *row_scales, int64_t n_row_scales, cudaStream_t s) {
     const int64_t nb = w->k / 256;
     const int most = m < RM_PASS ? m : RM_PASS;
-    int32_t rc = ensure_act(c, (size_t)nb * rm_slice_bytes(most));
+    int32_t rc = ensure_act(c, rm_image_bytes(most, nb));
     if (rc) return rc;
     RmParams p{};
     p.w = static_cast<const uint8_t *>(w->qs);
-    p.img = static_cast<const uint8_t *>(c->act);
     p.row_scales = row_scales;
     p.n_row_scales = row_scales ? n_row_scales : 0;
     p.n = w->n;
@@ -757,7 +847,10 @@ int32_t raw_mma_launch(Ctx *c, const Weight *w, const float *x, int64_t xst, int
     for (int t0 = 0; t0 < m; t0 += RM_PASS) {
         p.m = m - t0 < RM_PASS ? m - t0 : RM_PASS;
         p.y = y + (int64_t)t0 * yst;
-        RmStage sp{x + (int64_t)t0 * xst, xst, xsk, w->k, p.m, w->qt == GLLMK_QUANT_Q5_K, static_cast<uint8_t *>(c->act)};
+        uint8_t *img = static_cast<uint8_t *>(c->act), *rest = img + (size_t)nb * rm_slice_bytes(p.m);
+        p.img = img;
+        p.rest = rest;
+        RmStage sp{x + (int64_t)t0 * xst, xst, xsk, w->k, p.m, w->qt == GLLMK_QUANT_Q5_K, img, rest};
         GK_CUDA(c, launch_after(raw_mma_stage_kernel, !c->peer_waits, dim3((unsigned)nb, (unsigned)p.m), 64, 0, s, sp));
         switch (w->qt) {
             case GLLMK_QUANT_Q6_K: rc = rm_format<GLLMK_QUANT_Q6_K>(c, p, s); break;

@@ -450,6 +450,56 @@ def test_gemv_against_64_bit_product(K, gk, oracle, torch, name, n, k, m):
     w.free()
 
 
+def zero_weight_at(name, v, e):
+    """Makes element e (< 16) of every 256-element group decode to exactly 0 (Q5_K: its whole first sub-block)."""
+    if name == "q6_k":     # q - 32 = 0: low nibble 0, high pair 2
+        v[:, e] &= 0xF0
+        v[:, 128 + e] = (v[:, 128 + e] & 0xFC) | 2
+    elif name == "q5_k":   # scale and min of sub-block 0
+        v[:, 4] &= 0xC0
+        v[:, 8] &= 0xC0
+    elif name == "q8_k":
+        v[:, 4 + e] = 0
+    elif name == "q4_0":   # q - 8 = 0
+        v[::8, 2 + e] = (v[::8, 2 + e] & 0xF0) | 8
+    else:                  # q - 16 = 0: bit 4 from qh
+        v[::8, 6 + e] &= 0xF0
+        v[::8, 2 + e // 8] |= 1 << (e % 8)
+
+
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("n,k,m,big", [(512, 8 * 256, 1, 1e4), (500, 3 * 256, 3, 1e4), (512, 4 * 256, 6, 3e6), (300, 2 * 256, 11, 600.0), (256, 5 * 256, 16, 1e4)])
+def test_gemv_beside_an_outlier_the_weights_do_not_see(K, gk, oracle, torch, name, n, k, m, big):
+    """One element of each 256-block is `big` among N(0, 1) and its weights decode to 0: the products only see the small elements,
+    which a fixed point of the block's maximum alone would resolve to big * 1.2e-7.  Bar: the root mean square error over the
+    rows is no larger than what 16 bits per 32-element run give (step = run maximum / 32767, uniform rounding error).  Tokens
+    without outliers beside them give the same bits as alone."""
+    qt = qtype(gk, name)
+    rng = np.random.default_rng(n + m)
+    v = random_blocks(name, qt, n, k, 950 + m).reshape(-1, qt.block_bytes()).copy()
+    zero_weight_at(name, v, 5)
+    W = oracle_matrix(oracle, qt, v.reshape(-1), n, k).reshape(n, k).astype(np.float64)
+    assert not W[:, 5::256].any()
+    plain = rng.standard_normal((m, k)).astype(np.float32)
+    x = plain.copy()
+    hit = np.arange(0, m, 2)  # every other token
+    x[np.ix_(hit, np.arange(5, k, 256))] = np.float32(big)
+    w = K.upload(qt, n, k, v.reshape(-1))
+    y = K.gemv(w, torch.from_numpy(x).cuda()).cpu().numpy()
+    y_plain = K.gemv(w, torch.from_numpy(plain).cuda()).cpu().numpy()
+    y_t = K.gemv(w, torch.from_numpy(np.ascontiguousarray(x.T)).cuda(), ref_layout=True).cpu().numpy()
+    assert K.status() == 0
+    assert np.array_equal(y_t.T, y)
+    others = np.setdiff1d(np.arange(m), hit)
+    assert np.array_equal(y[others], y_plain[others])
+    step = np.abs(plain.reshape(m, k // 32, 32)).max(2) / 32767.0  # of the small elements: the run of the outlier, too, is held to it
+    for t in hit:
+        err = y[t] - x[t].astype(np.float64) @ W.T
+        s16 = np.sqrt(np.mean((W ** 2) @ (np.repeat(step[t], 32) ** 2) / 12.0))
+        assert np.sqrt(np.mean(err ** 2)) <= s16, (t, np.sqrt(np.mean(err ** 2)), s16)
+    w.free()
+
+
 @pytest.mark.parametrize("name", ["q4_0", "q5_0"])
 @pytest.mark.parametrize("k", [256 + 32, 512 - 32])
 def test_gemv_rows_of_other_lengths_stay_on_the_dp2a_kernel(K, gk, oracle, torch, name, k):
