@@ -63,11 +63,11 @@ int32_t ensure_host_word(Ctx *c) {
 int32_t ensure_dev_io(Ctx *c, size_t bytes) { return grow(c, &c->dev_io, &c->dev_io_bytes, bytes, false); }
 
 // ---- device memory of weights (device_pool.cuh) ----
-// Device buffers of a weight whose plane sizes are set: one allocation, the auxiliary plane behind the main one.
-static int32_t weight_buffers(Ctx *c, Weight *w, bool *waited) {
+// Device buffers of a weight whose plane sizes are set (on_device: its contents come from device memory): one allocation, the auxiliary plane behind the main one.
+static int32_t weight_buffers(Ctx *c, Weight *w, bool on_device, bool *waited) {
     const size_t aux_off = (w->qs_bytes + 255) & ~(size_t)255;
     w->alloc_bytes = aux_off + w->aux_bytes;
-    const cudaError_t e = pool_take(c->device, &w->alloc_bytes, &w->qs, waited);
+    const cudaError_t e = pool_take(c->device, &w->alloc_bytes, &w->qs, on_device, waited);
     if (e != cudaSuccess) return cuda_fail(c, e, "cudaMalloc(weight)");
     if (w->aux_bytes) w->aux = static_cast<char *>(w->qs) + aux_off;
     return GLLMK_STATUS_OK;
@@ -78,7 +78,7 @@ static int block_size_of(int qt, int mx) { return quant_format(qt, mx).block_siz
 static int block_bytes_of(int qt, int mx) { return quant_format(qt, mx).block_bytes; }
 
 // Creates the handle and its device buffers for an n x k matrix of type qt (no data yet).
-static int32_t weight_alloc(Ctx *c, int32_t qt, int64_t n, int64_t k, int32_t mx_block, float global, Weight **out, bool *waited) {
+static int32_t weight_alloc(Ctx *c, int32_t qt, int64_t n, int64_t k, int32_t mx_block, float global, bool on_device, Weight **out, bool *waited) {
     if (qt != GLLMK_QUANT_Q4K && qt != GLLMK_QUANT_Q8_0 && qt != GLLMK_QUANT_MXFP4 && qt != GLLMK_QUANT_NVFP4 && !raw_format(qt))
         return fail(c, GLLMK_STATUS_UNSUPPORTED, "unknown quant type %d", qt);
     if (qt == GLLMK_QUANT_MXFP4 && mx_block != 32)
@@ -120,7 +120,7 @@ static int32_t weight_alloc(Ctx *c, int32_t qt, int64_t n, int64_t k, int32_t mx
         w->qs_bytes = (size_t)w->n_pad * (w->k_pad / 2);
         w->aux_bytes = (size_t)w->n_pad * (w->k_pad / (qt == GLLMK_QUANT_NVFP4 ? 16 : 32));
     }
-    const int32_t rc = weight_buffers(c, w, waited);
+    const int32_t rc = weight_buffers(c, w, on_device, waited);
     if (rc) {
         delete w;
         return rc;
@@ -339,7 +339,7 @@ int32_t gllmk_weight_upload(gllmk_ctx ctx, int32_t quant_type, int64_t n, int64_
     DeviceGuard g(c->device);
     Weight *w = nullptr;
     bool waited = false;
-    int32_t rc = weight_alloc(c, quant_type, n, k, mx_block, global_scale, &w, &waited);
+    int32_t rc = weight_alloc(c, quant_type, n, k, mx_block, global_scale, src_on_device != 0, &w, &waited);
     if (rc) return rc;
     rc = weight_fill(c, w, blocks, scales, src_on_device != 0, waited);
     if (rc) { weight_destroy(w); return rc; }
@@ -588,7 +588,7 @@ static int32_t int8_weight_create(Ctx *c, int64_t n, int64_t k, const int8_t *b,
     w->qs_bytes = (size_t)w->n_pad * (size_t)w->k_pad;
     w->aux_bytes = (size_t)n * sizeof(int32_t);  // column sums of B (zero-point correction of the f32 activation path)
     bool waited = false;
-    int32_t rc = weight_buffers(c, w, &waited);
+    int32_t rc = weight_buffers(c, w, on_device, &waited);
     if (rc) {
         delete w;
         return rc;
@@ -1007,7 +1007,7 @@ static int32_t family_matmul(gllmk_ctx ctx, const uint8_t *wb, const float *inpu
     DeviceGuard g(c->device);
     Weight *w = nullptr;
     bool waited = false;
-    int32_t rc = weight_alloc(c, qt, (int64_t)m, (int64_t)k, 0, 1.0f, &w, &waited);
+    int32_t rc = weight_alloc(c, qt, (int64_t)m, (int64_t)k, 0, 1.0f, false, &w, &waited);
     if (rc) return rc;
     rc = weight_fill(c, w, wb, nullptr, false, waited);
     if (!rc) rc = matmul_host_impl(c, w, input, (int)n, output, true, nullptr, 0);
@@ -1036,7 +1036,7 @@ static int32_t gemm_kq_host(gllmk_ctx ctx, int32_t qt, const char *what, const v
     DeviceGuard g(c->device);
     Weight *w = nullptr;
     bool waited = false;
-    int32_t rc = weight_alloc(c, qt, (int64_t)n, (int64_t)k, 0, 1.0f, &w, &waited);
+    int32_t rc = weight_alloc(c, qt, (int64_t)n, (int64_t)k, 0, 1.0f, false, &w, &waited);
     if (rc) return rc;
     rc = weight_fill(c, w, weight, nullptr, false, waited);
     if (!rc) rc = matmul_host_impl(c, w, input, (int)m, output, false, scales, n_scales);

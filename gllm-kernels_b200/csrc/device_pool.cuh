@@ -6,7 +6,8 @@
 // therefore stay with the library, at most 128 MB per device, until the last context of the device is freed or an
 // allocation of a weight fails.
 // A buffer that is taken again may still be read by kernels its last owner launched, on any stream: the taker waits for the
-// device once (an upload from device memory has to anyway).
+// device once.  Only an upload from device memory takes one (it has to wait for the device anyway); an upload from the host
+// waits for nothing, so that it also works beside a stream capture of another thread, and its time is the bus's.
 // An allocation has the size that was asked for.  A buffer serves smaller requests too, as long as it is no more than an eighth
 // (or 64 KB) larger: activations whose token counts differ a little share buffers, and no weight holds much more than it needs.
 #pragma once
@@ -37,10 +38,11 @@ inline void pool_trim(int device) {
     p.blocks.clear();
     p.held = 0;
 }
-// A buffer of at least *bytes, which receives its size.  *waited: it is a freed one, and the device has been waited for.
-inline cudaError_t pool_take(int device, size_t *bytes, void **out, bool *waited) {
+// A buffer of at least *bytes, which receives its size.  reuse: it may be a freed one; *waited is set if it is (the device has been
+// waited for).
+inline cudaError_t pool_take(int device, size_t *bytes, void **out, bool reuse, bool *waited) {
     *out = nullptr;
-    {
+    if (reuse) {
         DevicePool &p = pool_of(device);
         std::lock_guard<std::mutex> l(p.mu);
         const size_t slack = *bytes / 8 > (size_t)65536 ? *bytes / 8 : (size_t)65536;

@@ -35,7 +35,7 @@ def run(tmp_path, body):
     (tmp_path / "t.cpp").write_text(
         '#include "device_pool.cuh"\n#include <cstdio>\nusing namespace gllmk;\n'
         '#define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\\n", __LINE__, #c); return 1; } } while (0)\n'
-        '#define TAKE(d, n, p, w) pool_take(d, n, p, w)\n'
+        '#define TAKE(d, n, p, w) pool_take(d, n, p, true, w)\n'
         'constexpr size_t MB = (size_t)1 << 20;\n'
         'int main() {\n' + body + '\nreturn 0;\n}\n')
     exe = tmp_path / "t"
@@ -83,3 +83,13 @@ def test_a_freed_buffer_serves_requests_of_about_its_size(tmp_path):
     CHECK(fake().used == used - 65 * MB);
     pool_trim(0);
     CHECK(pool_of(0).held == 0 && pool_of(0).blocks.empty());""")
+
+
+def test_an_upload_from_the_host_takes_no_freed_buffer(tmp_path):
+    """It would have to wait for the device, which no thread may do while another one captures a stream."""
+    run(tmp_path, r"""
+    pool_of(0).contexts = 1;
+    size_t n = 9 * MB; void *p, *q; bool waited = false;
+    CHECK(pool_take(0, &n, &p, true, &waited) == cudaSuccess);
+    pool_put(0, p, n);
+    CHECK(pool_take(0, &n, &q, false, &waited) == cudaSuccess && q != p && !waited && fake().waits == 0);""")

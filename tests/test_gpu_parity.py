@@ -596,3 +596,38 @@ def test_a_weight_takes_no_more_device_memory_than_it_holds(gk, K, torch, fmt, n
     assert took <= sum(w.info()["dev_bytes"] for w in ws) + 4 * (2 << 20)
     for w in ws:
         w.free()
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+def test_host_uploads_beside_another_threads_stream_capture(gk, K, torch, mode):
+    """A thread that loads a weight from host memory waits for its own copies only: while another thread captures a stream, a wait
+    for the device would be refused and spoil the capture, also when a freed buffer of the weight's size lies ready."""
+    import threading
+    qt, n, k = gk.QuantType.q8_0(), 1024, 1024
+    blocks = K.quantize(qt, torch.randn((n, k), device="cuda")).cpu().numpy()
+    w, x = K.upload(qt, n, k, blocks), torch.randn((2, k), device="cuda")
+    want, y = K.gemv(w, x).clone(), torch.zeros((2, n), device="cuda")
+    other = gk.GpuKernels(0)
+    other.upload(qt, n, k, blocks).free()
+    loaded, errors = [], []
+
+    def load():
+        try:
+            loaded.append(other.upload(qt, n, k, blocks))
+        except gk.GllmkError as e:
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream, capture_error_mode=mode):
+        K.gemv(w, x, y=y)
+        t = threading.Thread(target=load)
+        t.start()
+        t.join()
+    assert not errors
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    assert np.array_equal(other.unpack(loaded[0]), blocks)
+    other.close()
+    w.free()
