@@ -40,7 +40,7 @@ static int32_t grow(Ctx *c, void **p, size_t *have, size_t want, bool pinned) {
     }
     const size_t sz = (want + (1u << 20) - 1) & ~((size_t)(1u << 20) - 1);
     if (pinned) GK_CUDA(c, cudaMallocHost(p, sz));
-    else GK_CUDA(c, cudaMalloc(p, sz));
+    else GK_CUDA(c, device_malloc(c->device, p, sz));
     *have = sz;
     return GLLMK_STATUS_OK;
 }
@@ -145,7 +145,7 @@ static int32_t weight_fill(Ctx *c, Weight *w, const void *blocks, const void *sc
     void *stage = nullptr;
     if (!on_device) {
         const size_t off = (raw + 255) & ~(size_t)255;
-        GK_CUDA(c, cudaMalloc(&stage, off + sraw + 256));
+        GK_CUDA(c, device_malloc(c->device, &stage, off + sraw + 256));
         cudaError_t e = cudaMemcpyAsync(stage, blocks, raw, cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess && sraw)
             e = cudaMemcpyAsync(static_cast<char *>(stage) + off, scales, sraw, cudaMemcpyHostToDevice, c->stream);
@@ -229,7 +229,7 @@ int32_t gllmk_ctx_create(int32_t device, gllmk_ctx *out) {
     c->device = device;
     c->sm_count = prop.multiProcessorCount;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void **>(&c->status_dev), 16384) != cudaSuccess ||
+        device_malloc(device, reinterpret_cast<void **>(&c->status_dev), 16384) != cudaSuccess ||
         cudaMemset(c->status_dev, 0, 16384) != cudaSuccess) {
         (void)cudaGetLastError();
         if (c->stream) cudaStreamDestroy(c->stream);
@@ -380,7 +380,7 @@ int32_t gllmk_weight_unpack(gllmk_ctx ctx, gllmk_weight wh, void *blocks, void *
     }
     void *stage = nullptr;
     const size_t off = (raw + 255) & ~(size_t)255;
-    GK_CUDA(c, cudaMalloc(&stage, off + sraw + 256));
+    GK_CUDA(c, device_malloc(c->device, &stage, off + sraw + 256));
     int32_t rc = repack_unpack(c, w, stage, static_cast<char *>(stage) + off, c->stream);
     cudaError_t e = cudaSuccess;
     if (!rc) {
@@ -597,7 +597,7 @@ static int32_t int8_weight_create(Ctx *c, int64_t n, int64_t k, const int8_t *b,
     void *stage = nullptr;
     cudaError_t e = cudaSuccess;
     if (!on_device) {
-        e = cudaMalloc(&stage, (size_t)n * (size_t)k);
+        e = device_malloc(c->device, &stage, (size_t)n * (size_t)k);
         if (e == cudaSuccess) e = cudaMemcpyAsync(stage, b, (size_t)n * (size_t)k, cudaMemcpyHostToDevice, c->stream);
         if (e != cudaSuccess) {
             if (stage) cudaFree(stage);

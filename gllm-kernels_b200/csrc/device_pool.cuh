@@ -1,10 +1,10 @@
-// Device memory of weights.
+// Device memory of weights and scratch.
 //
 // cudaMalloc and cudaFree each cost tens to hundreds of microseconds and cudaFree waits for the device, which is nothing for a
 // model's weights but most of the time of a call whose activations are quantized and uploaded like a weight
 // (gllmk_gemm_fp4: W[14336, 4096] x 2048 tokens 850 - 1360 us, 600 of them here).  Freed weight buffers of up to 64 MB
-// therefore stay with the library, at most 128 MB per device, until the last context of the device is freed or an
-// allocation of a weight fails.
+// therefore stay with the library, at most 128 MB per device, until the last context of the device is freed or one of the
+// library's own allocations fails.
 // A buffer that is taken again may still be read by kernels its last owner launched, on any stream: the taker waits for the
 // device once.  Only an upload from device memory takes one (it has to wait for the device anyway); an upload from the host
 // waits for nothing, so that it also works beside a stream capture of another thread, and its time is the bus's.
@@ -38,6 +38,16 @@ inline void pool_trim(int device) {
     p.blocks.clear();
     p.held = 0;
 }
+// cudaMalloc on the current device, `device`; when memory is short, once more without the idle buffers.
+inline cudaError_t device_malloc(int device, void **out, size_t bytes) {
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        pool_trim(device);
+        e = cudaMalloc(out, bytes);
+    }
+    return e;
+}
 // A buffer of at least *bytes, which receives its size.  reuse: it may be a freed one; *waited is set if it is (the device has been
 // waited for).
 inline cudaError_t pool_take(int device, size_t *bytes, void **out, bool reuse, bool *waited) {
@@ -63,13 +73,7 @@ inline cudaError_t pool_take(int device, size_t *bytes, void **out, bool reuse, 
         else cudaFree(*out), *out = nullptr;
         return e;
     }
-    cudaError_t e = cudaMalloc(out, *bytes);
-    if (e == cudaErrorMemoryAllocation) {
-        (void)cudaGetLastError();
-        pool_trim(device);
-        e = cudaMalloc(out, *bytes);
-    }
-    return e;
+    return device_malloc(device, out, *bytes);
 }
 inline void pool_put(int device, void *ptr, size_t bytes) {
     if (!ptr) return;

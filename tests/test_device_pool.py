@@ -93,3 +93,24 @@ def test_an_upload_from_the_host_takes_no_freed_buffer(tmp_path):
     CHECK(pool_take(0, &n, &p, true, &waited) == cudaSuccess);
     pool_put(0, p, n);
     CHECK(pool_take(0, &n, &q, false, &waited) == cudaSuccess && q != p && !waited && fake().waits == 0);""")
+
+
+def test_any_allocation_may_claim_the_idle_buffers(tmp_path):
+    run(tmp_path, r"""
+    pool_of(0).contexts = 1;
+    void *p, *q;
+    for (int i = 0; i < 3; i++) { CHECK(cudaMalloc(&p, 40 * MB) == cudaSuccess); pool_put(0, p, 40 * MB); }
+    CHECK(pool_of(0).held == 120 * MB);
+    CHECK(device_malloc(0, &p, 380 * MB) == cudaSuccess && pool_of(0).held == 120 * MB);  // fits beside them
+    CHECK(device_malloc(0, &q, 100 * MB) == cudaSuccess && pool_of(0).held == 0);         // only without them
+    CHECK(device_malloc(0, &p, 512 * MB) == cudaErrorMemoryAllocation);""")
+
+
+def test_the_library_allocates_device_memory_in_one_place():
+    """cudaMalloc elsewhere would fail while idle weight buffers could be given back."""
+    import re
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")) and name != "device_pool.cuh":
+            with open(os.path.join(CSRC, name)) as f:
+                code = re.sub(r'//[^\n]*|"[^"\n]*"', "", f.read())
+                assert not re.search(r"\bcudaMalloc\s*\(", code), name
