@@ -95,7 +95,7 @@ struct Ctx {
     size_t dev_io_bytes = 0;
     cudaStream_t stream = nullptr;  // the context's own stream for host-pointer entry points
     void *host_word = nullptr;      // 8 KB of page-locked memory kernels leave small results for the host in (a scale, 1025 row offsets)
-    cudaEvent_t host_word_ready = nullptr;  // recorded behind the kernel that wrote it
+    cudaEvent_t host_word_ready = nullptr;  // recorded behind the kernels that wrote or used it
     // gllmk_matmul_host_batch: a second stream for the host <-> device copies (they run beside the products), events
     // for the hand-overs, and the instantiated graph of the last argument list that was seen twice
     cudaStream_t copy_stream = nullptr;

@@ -347,12 +347,9 @@ int32_t quantize_launch(Ctx *c, int32_t qt, const float *x, int64_t rows, int64_
     } else if (qt == GLLMK_QUANT_NVFP4) {
         const bool given = *global_scale > 0.0f;
         if (!given) {
-            // the scale goes to the host as soon as the first pass has it; the encoder runs under the host's wait and the
-            // caller's next steps
             int32_t rc = ensure_host_word(c);
             if (!rc) rc = amax_launch(c, x, 1, (int64_t)count, (int64_t)count, static_cast<float *>(c->host_word), s);
             if (rc) return rc;
-            GK_CUDA(c, cudaEventRecord(c->host_word_ready, s));
         }
         const size_t units = count / 8;
         const unsigned grid = (unsigned)((units + 256 * QF_UNITS - 1) / (256 * QF_UNITS));
@@ -362,6 +359,9 @@ int32_t quantize_launch(Ctx *c, int32_t qt, const float *x, int64_t rows, int64_
         else GK_CUDA(c, launch_after(quantize_nvfp4_kernel, true, dim3(grid), 256, 0, s, x, vec, out, &amax_out(c)->global, 0.0f, units));
         GK_CUDA(c, cudaGetLastError());
         if (!given) {
+            // the call returns the scale, so it waits; and it waits for the blocks, not for the first pass alone: whoever holds the
+            // scale may read them on any stream, and the encoder reads the context's small scratch, which the next call rewrites
+            GK_CUDA(c, cudaEventRecord(c->host_word_ready, s));
             GK_CUDA(c, cudaEventSynchronize(c->host_word_ready));
             *global_scale = *static_cast<volatile float *>(c->host_word);
         }

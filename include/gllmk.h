@@ -490,7 +490,8 @@ GLLMK_API int32_t gllmk_dequant_gguf(gllmk_ctx ctx, int32_t quant_type, const ui
  * these formats (its only quantizer is per-tensor amax/127, src/compiler/quant_convert.rs:17-31);
  * these are this library's own, used for NVFP4 activations and to make synthetic weights.
  * MXFP4 writes the split form (blocks + scales).  NVFP4: *global_scale > 0 is used as given,
- * otherwise amax/(6*448) of the whole input is computed, used and written back. */
+ * otherwise amax/(6*448) of the whole input is computed, used and written back, and the call returns when the
+ * blocks are complete. */
 GLLMK_API int32_t gllmk_quantize(gllmk_ctx ctx, int32_t quant_type, const float *x_dev, int64_t rows, int64_t k,
                        int32_t mx_block, void *blocks_dev, void *scales_dev, float *global_scale, void *stream);
 

@@ -631,3 +631,23 @@ def test_host_uploads_beside_another_threads_stream_capture(gk, K, torch, mode):
     assert np.array_equal(other.unpack(loaded[0]), blocks)
     other.close()
     w.free()
+
+
+@pytest.mark.parametrize("rows", [1, 4096])
+def test_nvfp4_quantize_returns_with_complete_blocks(gk, K, torch, rows):
+    """The call that works out the global scale waits for it, and returns with the blocks written: another stream may read them
+    at once, and another call on another stream may follow."""
+    k = 14336
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    xs = [torch.randn((rows, k), device="cuda", generator=gen) * (10.0 ** i) for i in range(4)]
+    want = [K.quantize(gk.QuantType.nvfp4(), x) for x in xs]
+    torch.cuda.synchronize()
+    writers, reader, got = [torch.cuda.Stream(), torch.cuda.Stream()], torch.cuda.Stream(), []
+    for i, x in enumerate(xs):
+        with torch.cuda.stream(writers[i % 2]):
+            blocks, scale = K.quantize(gk.QuantType.nvfp4(), x)
+        with torch.cuda.stream(reader):
+            got.append((blocks.clone(), scale, blocks))
+    torch.cuda.synchronize()
+    for (b, s), (copy, scale, _) in zip(want, got):
+        assert scale == s and torch.equal(copy, b)
