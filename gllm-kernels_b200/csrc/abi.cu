@@ -770,7 +770,9 @@ static int32_t matmul_host_impl(Ctx *c, const Weight *w, const float *x_host, in
     // own page-locked area serves the others the same way (W[11008, 4096]: Q8_0 x 8 tokens 54 -> 43 us per call, Q6_K 54 -> 46, one token
     // 34 -> 31; a 0.9 MB result is better copied, 65 against 68 us).  A token's rows lie side by side.
     const bool decode = ref_layout || sb || m_t <= GLLMK_GEMM_GEMV_MAX_M || raw_format(w->qt);
-    const bool zero_copy_y = decode && m_t <= GLLMK_GEMV_MAX_M && (!ref_layout || m_t == 1) && yb <= (size_t)512 * 1024;
+    // Not in place: a product that converts its activations as it goes ("gemv_fuse") still reads x while other CTAs store.
+    const bool apart = y_host + (size_t)m_t * n_w <= x_host || x_host + (size_t)m_t * k <= y_host;
+    const bool zero_copy_y = decode && apart && m_t <= GLLMK_GEMV_MAX_M && (!ref_layout || m_t == 1) && yb <= (size_t)512 * 1024;
     float *yd = zero_copy_y ? (y_pinned ? static_cast<float *>(const_cast<void *>(y_alias)) : reinterpret_cast<float *>(pin + yo))
                             : reinterpret_cast<float *>(dev + yo);
     const float *sd = sb ? reinterpret_cast<const float *>(dev + so) : nullptr;

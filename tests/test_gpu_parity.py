@@ -651,3 +651,23 @@ def test_nvfp4_quantize_returns_with_complete_blocks(gk, K, torch, rows):
     torch.cuda.synchronize()
     for (b, s), (copy, scale, _) in zip(want, got):
         assert scale == s and torch.equal(copy, b)
+
+
+@pytest.mark.parametrize("fuse", [0, 2])
+def test_matmul_host_in_place_on_page_locked_memory(gk, K, oracle, torch, fuse):
+    """The result over the activations, in the caller's page-locked buffer; with "gemv_fuse" the product's CTAs read their
+    activations while others have finished theirs."""
+    n = k = 4096
+    W = (np.random.default_rng(5).standard_normal((n, k)) * 0.02).astype(np.float32)
+    w = K.upload(gk.QuantType.q4k(), n, k, oracle.quantize_q4_k(W))
+    x = np.random.default_rng(6).standard_normal((1, k)).astype(np.float32)
+    K.set("gemv_fuse", fuse)
+    try:
+        want = K.matmul_host(w, x)
+        buf = torch.empty((1, k), dtype=torch.float32, pin_memory=True).numpy()
+        for _ in range(5):
+            buf[:] = x
+            assert np.array_equal(K.matmul_host(w, buf, out=buf), want)
+    finally:
+        K.set("gemv_fuse", 0)
+    w.free()
