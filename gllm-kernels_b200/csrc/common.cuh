@@ -116,7 +116,7 @@ struct Ctx {
     int64_t gemm_i8_pair = 1;   // W8A8 GEMM with m > 128 on CTA pairs (cta_group::2, persistent, two accumulators): 0 never,
                                 // 1 when the estimate favours it, 2 always
     int64_t gemm_raw_slots = 0;  // weight-only GEMM: raw super-chunk ring depth (0 = chosen by the shared-memory plan)
-    int64_t gemm_pdl = 1;        // weight-only GEMM launched programmatically behind its activation staging kernel
+    int64_t gemm_pdl = 1;        // weight-only GEMM and its activation staging kernel launched programmatically
     int64_t raw_gemv_mma = 1;    // Q4_0 / Q5_0 rows of whole 256-element groups: 0 = the dp2a kernel (the other row-major formats have one kernel)
     int64_t gemm_row_tiles = 0;  // weight-only GEMM: row tiles per CTA (0 = estimated, 1, 2)
     // The context has launched a wait for another rank.  What is queued behind one must not hold the SMs for as long as it lasts

@@ -1018,7 +1018,7 @@ static int32_t gemm_groups_chunk(Ctx *c, const Weight *const *ws, int ng, const 
     int32_t rc = ensure_act(c, (size_t)nimg * nks * WQ_TILE);
     if (rc) return rc;
     p.xt = static_cast<const uint8_t *>(c->act);
-    GK_CUDA(c, launch_after(stage_act_kernel, !c->peer_waits, dim3((unsigned)nks, (unsigned)nimg), 256, 0, s, a, a_bf16, lda, (int64_t)w->k,
+    GK_CUDA(c, launch_after(stage_act_kernel, c->gemm_pdl != 0 && !c->peer_waits, dim3((unsigned)nks, (unsigned)nimg), 256, 0, s, a, a_bf16, lda, (int64_t)w->k,
                             static_cast<uint8_t *>(c->act), imgs, a_up, wq_quads(fmt) ? 1 : 0));
     dim3 grid((unsigned)ntiles, (unsigned)((row_tiles + mt - 1) / mt));
     // Tail split: the last, partly filled wave of tiles — the only one, when there are fewer tiles than SMs — is cut along

@@ -804,7 +804,7 @@ int32_t rm_pass(Ctx *c, RmParams &p, cudaStream_t s) {
     if (rc) return rc;
     p.partial = static_cast<float *>(c->red);
     p.counters = static_cast<int *>(c->cnt);
-    GK_CUDA(c, launch_after(raw_mma_gemv_kernel<QT, NG>, true, dim3((unsigned)ctas), RM_WARPS * 32, rm_smem_bytes<QT>(p.m, p.stages), s, p));
+    GK_CUDA(c, launch_after(raw_mma_gemv_kernel<QT, NG>, c->gemv_pdl != 0, dim3((unsigned)ctas), RM_WARPS * 32, rm_smem_bytes<QT>(p.m, p.stages), s, p));
     return GLLMK_STATUS_OK;
 }
 
@@ -851,7 +851,7 @@ int32_t raw_mma_launch(Ctx *c, const Weight *w, const float *x, int64_t xst, int
         p.img = img;
         p.rest = rest;
         RmStage sp{x + (int64_t)t0 * xst, xst, xsk, w->k, p.m, w->qt == GLLMK_QUANT_Q5_K, img, rest};
-        GK_CUDA(c, launch_after(raw_mma_stage_kernel, !c->peer_waits, dim3((unsigned)nb, (unsigned)p.m), 64, 0, s, sp));
+        GK_CUDA(c, launch_after(raw_mma_stage_kernel, c->gemv_pdl != 0 && !c->peer_waits, dim3((unsigned)nb, (unsigned)p.m), 64, 0, s, sp));
         switch (w->qt) {
             case GLLMK_QUANT_Q6_K: rc = rm_format<GLLMK_QUANT_Q6_K>(c, p, s); break;
             case GLLMK_QUANT_Q5_K: rc = rm_format<GLLMK_QUANT_Q5_K>(c, p, s); break;

@@ -163,7 +163,7 @@ GLLMK_API int32_t gllmk_ctx_status(gllmk_ctx ctx, int32_t *device_status);
  * 0 automatic, 1 never, n into n), "gemm_row_tiles" (prefill GEMM, 128-row weight tiles per CTA: 0 estimated, 1, 2),
  * "gemm_raw_slots" (prefill GEMM, depth of the raw weight ring: 0 = what the shared-memory plan gives),
  * "raw_gemv_mma" (decode products of Q4_0 / Q5_0 rows of whole 256-element groups: 1 default, 0 the dp2a kernel),
- * "gemm_pdl" (prefill GEMM launched programmatically behind its activation staging kernel: 1 default, 0 plain launch), "peer_wait_spins" (how many times a wait on another GPU's flag probes it
+ * "gemm_pdl" (prefill GEMM and its activation staging kernel launched programmatically behind what precedes them: 1 default, 0 plain launches), "peer_wait_spins" (how many times a wait on another GPU's flag probes it
  * before it gives up with status 31; default 2^22, about a second), "inject_give_up" (testing aid, host side
  * only: leaves the context as a kernel that gave up a wait with that status code would — word set, arrival
  * counters dirty — without making any kernel wait). */
