@@ -16,6 +16,7 @@
 //     y += d * sum_sub sc_sub * (q . x)_sub  -  dmin * sum_sub m_sub * (sum x)_sub
 // Q8_0 per 32-block and row (classic.rs:870-881):  y += d * (q . x)
 #include "common.cuh"
+#include "share_plan.cuh"
 
 namespace gllmk {
 
@@ -864,17 +865,11 @@ struct GemvGrid {
     int per_cta, rem;
 };
 template <int FMT, int NT>
-static cudaError_t gemv_grid(Ctx *c, int m, int64_t nsuper, GemvGrid *g) {
+static cudaError_t gemv_grid(Ctx *c, int m, int64_t nsuper, int nk, GemvGrid *g) {
     cudaError_t e = gemv_occupancy<FMT, NT>(c->device, m, gemv_smem_bytes<FMT>(m), &g->per_sm);
     if (e != cudaSuccess) return e;
     if (c->gemv_ctas_per_sm > 0 && c->gemv_ctas_per_sm < g->per_sm) g->per_sm = (int)c->gemv_ctas_per_sm;
-    g->ctas = (int64_t)c->sm_count * g->per_sm;
-    if (g->ctas > nsuper) g->ctas = nsuper;
-    // few super-chunks per CTA: no more CTAs than the longest share needs; their tiles have fewer shares to write, count and add up
-    // (W[11008, 4096] Q4_K, 1376 super-chunks on 444 or 344 CTAs: one token 13.1 -> 11.8 us; with two super-chunks in a few CTAs only —
-    // W[7168, 2048], 448 on 444 — or one group of columns the larger grid is the faster one, 9.3 against 10.1 us at five tokens)
-    const int64_t longest = (nsuper + g->ctas - 1) / g->ctas;
-    if (longest <= 4 && (longest > 2 || (NT > 1 && nsuper * 10 >= g->ctas * 11))) g->ctas = (nsuper + longest - 1) / longest;
+    g->ctas = decode_ctas(nsuper, (int64_t)c->sm_count * g->per_sm, g->per_sm, nk, NT > 1);
     g->per_cta = (int)(nsuper / g->ctas);
     g->rem = (int)(nsuper % g->ctas);
     return cudaSuccess;
@@ -887,7 +882,7 @@ static cudaError_t gemv_fuse_plan(Ctx *c, int m, int64_t ntg, int nk, int *slice
     *slices = 0;
     if (!c->gemv_fuse || m > 4) return cudaSuccess;
     GemvGrid g;
-    cudaError_t e = gemv_grid<FMT, 1>(c, m, ntg * nk, &g);
+    cudaError_t e = gemv_grid<FMT, 1>(c, m, ntg * nk, nk, &g);
     if (e != cudaSuccess) return e;
     const int share = g.per_cta + (g.rem ? 1 : 0);
     const int nsl = share < nk ? share : nk;
@@ -911,7 +906,7 @@ template <int FMT, int NT>
 static cudaError_t configure_and_launch(Ctx *c, GemvParams &p, int64_t ntg, cudaStream_t s, int32_t *rc_out, int fuse_slices) {
     p.nsuper = ntg * p.nk;
     GemvGrid g;
-    cudaError_t e = gemv_grid<FMT, NT>(c, p.m, p.nsuper, &g);
+    cudaError_t e = gemv_grid<FMT, NT>(c, p.m, p.nsuper, p.nk, &g);
     if (e != cudaSuccess) return e;
     p.per_cta = g.per_cta;
     p.rem = g.rem;

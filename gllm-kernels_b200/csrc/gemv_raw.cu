@@ -28,6 +28,7 @@
 //   Q5_0             54 (67)  3.0 TB/s   72          98 (590)          21
 // With a wide block in every CTA 1.7 times that (geometric mean); the flags and scales of the second slices cost the others 3 %.
 #include "common.cuh"
+#include "share_plan.cuh"
 
 namespace gllmk {
 
@@ -786,14 +787,7 @@ int32_t rm_pass(Ctx *c, RmParams &p, cudaStream_t s) {
     GK_CUDA(c, (rm_plan<QT, NG>(c->device, p.m, &per_sm, &p.stages)));
     if (c->gemv_ctas_per_sm > 0 && c->gemv_ctas_per_sm < per_sm) per_sm = (int)c->gemv_ctas_per_sm;
     const int64_t groups = (p.n + RM_ROWS - 1) / RM_ROWS, units = groups * p.nb;
-    int64_t ctas = (int64_t)c->sm_count * per_sm;
-    if (ctas > units) ctas = units;
-    // few units per CTA: no more CTAs than the longest share needs — 512 units on 444 CTAs take as long as on 256 CTAs of two, whose
-    // tiles have half the shares to write, count and add up (W[4096, 4096]: 13.1 -> 12.2 us at 5 tokens, W[11008, 4096], four units:
-    // 15.7 -> 14.8).  With one or two tokens and two units, or two units in a few CTAs only, the larger
-    // grid is the faster one (10.2 against 10.6 us)
-    const int64_t longest = (units + ctas - 1) / ctas;
-    if (longest <= 4 && (longest > 2 || (NG > 1 && units * 10 >= ctas * 11))) ctas = (units + longest - 1) / longest;
+    const int64_t ctas = decode_ctas(units, (int64_t)c->sm_count * per_sm, per_sm, p.nb, NG > 1);
     if (units / ctas > 0x3fffffff) return fail(c, GLLMK_STATUS_INVALID_ARG, "gemv: matrix too large");
     p.per_cta = (int)(units / ctas);
     p.rem = (int)(units % ctas);
