@@ -52,9 +52,11 @@ enum {
     GLLMK_QUANT_NVFP4 = 4, /* QuantType::Nvfp4   64 el /  36 B  (src/quant.rs:366-371) */
     GLLMK_QUANT_INT8 = 5,  /* plain s8 matrix of the W8A8 path (gllmk_int8_weight_upload); not a block format */
     /* The other GGUF formats of the reference's CPU quant path.  Kept on the device as the reference stores them
-     * (Q6_K in 224-byte slots) and served by a streaming CUDA-core integer-dot GEMV (f32 activations and outputs,
-     * any m) plus decode / gather / unpack; gllmk_gemm with bf16 operands, gllmk_gemm_grouped, gllmk_gemv_allgather and gllmk_ffn_decode
-     * answer GLLMK_STATUS_UNSUPPORTED for them. */
+     * (Q6_K in 224-byte slots) and served by a streaming GEMV on the integer tensor core (f32 activations and outputs, any m; Q4_0 /
+     * Q5_0 rows that are not whole groups of 256 elements: CUDA-core integer dot products) plus decode / gather / unpack.  Q6_K,
+     * Q5_K and, with k a multiple of 256, Q4_0 / Q5_0 also have a place in gllmk_gemm, gllmk_gemm_grouped and gllmk_ffn_prefill.
+     * gllmk_gemv_allgather, gllmk_gemv_exchange and gllmk_ffn_decode answer GLLMK_STATUS_UNSUPPORTED for all of them, and so does
+     * gllmk_gemm with bf16 operands where only the GEMV serves the shape. */
     GLLMK_QUANT_Q6_K = 6,  /* QuantType::Q6K    256 el / 210 B  (src/quant.rs:143-148) */
     GLLMK_QUANT_Q5_K = 7,  /* QuantType::Q5K    256 el / 176 B  (src/quant.rs:132-138) */
     GLLMK_QUANT_Q4_0 = 8,  /* QuantType::Q4_0    32 el /  18 B  (src/quant.rs:254-257) */
@@ -342,10 +344,11 @@ GLLMK_API int32_t gllmk_exchange_wait(gllmk_ctx ctx, void *flags_local, int32_t 
  * evaluation.  a and its rows must be 16-byte aligned.  With f32 in and out and
  * m <= GLLMK_GEMM_GEMV_MAX_M the call is one pass of the decode kernel (gllmk_gemv), which is faster
  * there and meets its tighter bound (from 17 tokens on the tensor-core kernel is the faster one:
- * W[28672, 8192] Q4_K at m = 32: 80 us against 113 us as two decode passes).  Of the other GGUF formats Q6_K and Q5_K
- * have a place in this kernel (Q6_K: more than 8 tokens, up to 8 its batch GEMV; Q5_K: 2 tokens and more; f32 only below),
- * and so have Q4_0 and Q5_0 when k is a multiple of 256 (2 tokens and more); Q8_K, and Q4_0 / Q5_0 with another k, run the
- * streaming GEMV over token tiles and take f32 only. */
+ * W[28672, 8192] Q4_K at m = 32: 57 us against 113 us as two decode passes).  Of the other GGUF formats Q6_K and Q5_K
+ * have a place in this kernel (Q6_K: more than 8 tokens, up to 8 its GEMV, f32 only; Q5_K: 2 tokens and more), and so have
+ * Q4_0 and Q5_0 when k is a multiple of 256 (2 tokens and more); with 16-byte aligned f32 in and f32 out the last three run up
+ * to GLLMK_GEMM_GEMV_MAX_M tokens on the GEMV.  Q8_K, and Q4_0 / Q5_0 with another k, run the streaming GEMV over token
+ * tiles and take f32 only. */
 #define GLLMK_GEMM_GEMV_MAX_M 16
 GLLMK_API int32_t gllmk_gemm(gllmk_ctx ctx, gllmk_weight w, const void *a_dev, int32_t a_dtype, int64_t lda, int32_t m,
                              void *y_dev, int32_t y_dtype, int64_t ldy, void *stream);

@@ -1,8 +1,8 @@
 """Decode kernels under activations that are NOT standard normal, and the failure path of the bounded waits.
 
 The decode kernels do not multiply in f32: every token's activations are re-expressed once per call as small
-integer digits with one scale per k-block (Q4_K / Q8_0: two int8 digits per 256; the other GGUF formats: s16 per
-32; FP4 weights: eight E2M1 digits per scale block), so the error of a product grows with amax / rms of a block.
+integer digits with one scale per k-block (Q4_K / Q8_0: two int8 digits per 256; the other GGUF formats: three, and three more
+where a 256-block spans more than 8 bits; FP4 weights: eight E2M1 digits per scale block), so the error of a product grows with amax / rms of a block.
 These cases plant what LLM hidden states and silu(gate) * up really contain — heavy tails and one huge outlier in
 every block — and hold the same 2e-3 bar as the N(0, 1) cases.  Worst case of the two-digit form (one element
 dominating every 256-block): about 6.5e-4.
