@@ -12,7 +12,7 @@
 //     store it in tensor memory (tcgen05.st), from where the MMA takes operand A.  As a swizzled tile in shared
 //     memory it was written and read there once more, 256 of the ~480 cycles of shared-memory traffic that an A tile
 //     of a small batch cost (~750 at 256 tokens, against 540 of tensor-core time), and needed a proxy fence of ~150:
-//     W[28672, 8192] Q4_K x 33 tokens 80 us, now 59; x 512 tokens 201 us, now 195;
+//     W[28672, 8192] Q4_K x 33 tokens 80 us, now 58; x 128 tokens 90 us, now 65 (back to back in a CUDA graph);
 //   * the activations were converted once per call to fp16 tile images (stage_act_kernel), so operand B
 //     of a k-step is one or two bulk copies of 16 KB;
 //   * one elected thread issues tcgen05.mma (kind::f16, f32 accumulate in TMEM); tcgen05.commit hands the
