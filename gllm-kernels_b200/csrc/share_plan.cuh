@@ -28,7 +28,7 @@ inline int64_t decode_ctas(int64_t units, int64_t ctas, int per_sm, int64_t nb, 
     const int64_t longest = (units + ctas - 1) / ctas;
     bool fewer = false;
     if (longest == 4) fewer = nb % 12 != 0 && (per_sm < 3 || (nb % 4 == 0 && !(several && nb >= 16)));  // (shares of three and four both end at 12)
-    else if (longest == 3) fewer = per_sm < 3 && nb >= 16 && units * 10 >= ctas * 23;
+    else if (longest == 3) fewer = per_sm < 3 && nb >= 16 && units * 4 >= ctas * 9;
     else if (longest == 2) fewer = several && nb >= 16 && units * 10 >= ctas * 11;
     return fewer ? (units + longest - 1) / longest : ctas;
 }
