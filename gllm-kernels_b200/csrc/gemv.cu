@@ -869,7 +869,7 @@ static cudaError_t gemv_grid(Ctx *c, int m, int64_t nsuper, int nk, GemvGrid *g)
     cudaError_t e = gemv_occupancy<FMT, NT>(c->device, m, gemv_smem_bytes<FMT>(m), &g->per_sm);
     if (e != cudaSuccess) return e;
     if (c->gemv_ctas_per_sm > 0 && c->gemv_ctas_per_sm < g->per_sm) g->per_sm = (int)c->gemv_ctas_per_sm;
-    g->ctas = decode_ctas(nsuper, (int64_t)c->sm_count * g->per_sm, g->per_sm, nk, NT > 1);
+    g->ctas = decode_ctas(nsuper, (int64_t)c->sm_count * g->per_sm, g->per_sm, nk, NT > 1, true);
     g->per_cta = (int)(nsuper / g->ctas);
     g->rem = (int)(nsuper % g->ctas);
     return cudaSuccess;

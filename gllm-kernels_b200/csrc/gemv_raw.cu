@@ -787,7 +787,7 @@ int32_t rm_pass(Ctx *c, RmParams &p, cudaStream_t s) {
     GK_CUDA(c, (rm_plan<QT, NG>(c->device, p.m, &per_sm, &p.stages)));
     if (c->gemv_ctas_per_sm > 0 && c->gemv_ctas_per_sm < per_sm) per_sm = (int)c->gemv_ctas_per_sm;
     const int64_t groups = (p.n + RM_ROWS - 1) / RM_ROWS, units = groups * p.nb;
-    const int64_t ctas = decode_ctas(units, (int64_t)c->sm_count * per_sm, per_sm, p.nb, NG > 1);
+    const int64_t ctas = decode_ctas(units, (int64_t)c->sm_count * per_sm, per_sm, p.nb, NG > 1, false);
     if (units / ctas > 0x3fffffff) return fail(c, GLLMK_STATUS_INVALID_ARG, "gemv: matrix too large");
     p.per_cta = (int)(units / ctas);
     p.rem = (int)(units % ctas);

@@ -5,7 +5,8 @@
 
 namespace gllmk {
 
-// `ctas` resident CTAs (per_sm on an SM), several = more than one group of MMA columns.  With few units per CTA the shares differ by one
+// `ctas` resident CTAs (per_sm on an SM), several = more than one group of MMA columns, tiled = gemv.cu's kernel (gemv_raw.cu's
+// otherwise).  With few units per CTA the shares differ by one
 // unit in two or three, and a grid no larger than the longest share needs takes as many steps with fewer flushes — where its shares end
 // at a row group's end.  Where they do not, or where the resident grid's do, the larger grid is the faster one: the rest of its CTAs
 // leave their bandwidth to the others.  Time on the smaller grid over time on the larger one, one / five tokens, rows of nb blocks:
@@ -23,11 +24,11 @@ namespace gllmk {
 //   longest share 2 (512 on 444), five tokens
 //     Q4_K / Q5_K                          1.07/1.12 1.06/1.07 1.02/1.02 1.00/1.00  .98/1.00  .99/.97   .95/.93   .92/.91   .98/.92   .85/.81
 // (with one column group 1.0 - 1.14).  Five units and more: slower by up to 30 % but for eight that end at a row group's end.
-inline int64_t decode_ctas(int64_t units, int64_t ctas, int per_sm, int64_t nb, bool several) {
+inline int64_t decode_ctas(int64_t units, int64_t ctas, int per_sm, int64_t nb, bool several, bool tiled) {
     if (ctas > units) ctas = units;
     const int64_t longest = (units + ctas - 1) / ctas;
     bool fewer = false;
-    if (longest == 4) fewer = nb % 12 != 0 && (per_sm < 3 || (nb % 4 == 0 && !(several && nb >= 16)));  // (shares of three and four both end at 12)
+    if (longest == 4) fewer = nb % 12 != 0 && (per_sm < 3 || (nb % 4 == 0 && !(tiled && several && nb >= 16)));  // (shares of three and four both end at 12)
     else if (longest == 3) fewer = per_sm < 3 && nb >= 16 && units * 4 >= ctas * 9;
     else if (longest == 2) fewer = several && nb >= 16 && units * 10 >= ctas * 11;
     return fewer ? (units + longest - 1) / longest : ctas;
